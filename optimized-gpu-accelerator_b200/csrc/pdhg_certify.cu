@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -27,6 +28,7 @@
 #include "pdhg_cert.h"
 #include "pdhg_host_common.h"
 #include "pdhg_kernels.cuh"
+#include "pdhg_ordered.cuh"
 
 namespace b2p {
 
@@ -183,18 +185,35 @@ __global__ void __launch_bounds__(kBlock) k_ns_cols(int32_t m, int32_t n, CsrVie
   terms[static_cast<int64_t>(b) * (m + n) + m + j] = term;
 }
 
-// One thread per case: lb = 0; lb = add_down(lb, term) in index order (rows, then columns).
-__global__ void k_ns_sum(int32_t k, int64_t len, const double* __restrict__ terms, const int32_t* __restrict__ inf_terms,
-                         double* __restrict__ bound) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= k) return;
-  const double* tb = terms + static_cast<int64_t>(b) * len;
-  double lb = 0;
-  for (int64_t q = 0; q < len; ++q) {
-    const double v = tb[q];
-    if (!isnan(v)) lb = ns::add_down(lb, v);
-  }
-  bound[b] = inf_terms[b] > 0 ? -INFINITY : lb;
+// One block per case: lb = 0; lb = add_down(lb, term) in index order (rows,
+// then columns).  add_down is the hardware's downward-rounded addition but
+// for an overflow (which it reports as the round-to-nearest infinity) and the
+// sign of a zero sum, so a chunk is folded with __dadd_rd, its largest partial
+// sum watched beside the chain, and folded again step by step if that left
+// the finite range; a marked column (NaN) adds nothing.
+__global__ void __launch_bounds__(kOrderedThreads) k_ns_sum(int64_t len, const double* __restrict__ terms,
+                                                            const int32_t* __restrict__ inf_terms,
+                                                            double* __restrict__ bound) {
+  const int b = blockIdx.x;
+  const double* tb = terms + b * len;
+  const double lb = ordered_sum(
+      len,
+      [&](int64_t i) {
+        const double v = tb[i];
+        return isnan(v) ? 0.0 : v;
+      },
+      [](double s, const double* term, int count) {
+        double t = s, top = 0.0;
+#pragma unroll 16
+        for (int i = 0; i < count; ++i) {
+          t = __dadd_rd(t, term[i]);
+          top = fmax(top, fabs(t));
+        }
+        if (top < DBL_MAX && !isnan(t)) return t == 0.0 ? 0.0 : t;
+        for (int i = 0; i < count; ++i) s = ns::add_down(s, term[i]);
+        return s;
+      });
+  if (threadIdx.x == 0) bound[b] = inf_terms[b] > 0 ? -INFINITY : lb;
 }
 
 void enqueue_safe_bound(cudaStream_t s, int32_t m, int32_t n, int32_t k, CsrView AT, const double* y, const double* c,
@@ -206,7 +225,7 @@ void enqueue_safe_bound(cudaStream_t s, int32_t m, int32_t n, int32_t k, CsrView
   if (n)
     k_ns_cols<<<dim3((n + kBlock - 1) / kBlock, k), kBlock, 0, s>>>(m, n, AT, yp, c, lo, up, terms, stats,
                                                                     inf_terms);
-  k_ns_sum<<<(k + 127) / 128, 128, 0, s>>>(k, static_cast<int64_t>(m) + n, terms, inf_terms, bound);
+  k_ns_sum<<<k, kOrderedThreads, 0, s>>>(static_cast<int64_t>(m) + n, terms, inf_terms, bound);
   B2P_CUDA(cudaGetLastError());
 }
 

@@ -28,6 +28,7 @@
 
 #include "pdhg_host_common.h"
 #include "pdhg_kernels.cuh"
+#include "pdhg_ordered.cuh"
 #include "pdhg_prepare.h"
 #include "pdhg_restart.h"
 #include "pdhg_scale.cuh"
@@ -248,8 +249,8 @@ __global__ void k_offset_segments(const int64_t* __restrict__ seg, const int32_t
 // ---- ||A|| of every LP at once (powerIteration, src/pdhg/pdhg.cpp:404-422) ----
 // The block-diagonal A x and A^T y are CSR row sums in increasing column
 // order -- the addition order of the reference's scatter products -- and each
-// LP's ||z|| is summed by one thread in index order, so every LP's estimate is
-// bit-identical to its own sequential power iteration.
+// LP's ||z|| is summed in index order (pdhg_ordered.cuh), so every LP's
+// estimate is bit-identical to its own sequential power iteration.
 
 // x_j = 1 / sqrt(n_b) for the columns of LP b; LPs without entries are done
 // from the start with ||A|| = 1.
@@ -268,14 +269,22 @@ __global__ void k_pi_init(int32_t N, int32_t K, const int32_t* __restrict__ cins
   }
 }
 
-// One thread per LP: nz = sqrt(sum z_j^2) in index order; nz == 0 ends the
+// One block per LP: nz = sqrt(sum z_j^2) in index order; nz == 0 ends the
 // LP's iteration with ||A|| = 1, else s = sqrt(nz).
-__global__ void k_pi_norm(int32_t K, const int32_t* __restrict__ coff, const double* __restrict__ z,
-                          int32_t* __restrict__ done, double* __restrict__ nz_out, double* __restrict__ s) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= K || done[b]) return;
-  double acc = 0.0;
-  for (int32_t j = coff[b]; j < coff[b + 1]; ++j) acc = __dadd_rn(acc, __dmul_rn(z[j], z[j]));
+__global__ void __launch_bounds__(kOrderedThreads) k_pi_norm(const int32_t* __restrict__ coff,
+                                                             const double* __restrict__ z, int32_t* __restrict__ done,
+                                                             double* __restrict__ nz_out, double* __restrict__ s) {
+  const int b = blockIdx.x;
+  if (done[b]) return;
+  const double* zb = z + coff[b];
+  const double acc = ordered_sum(
+      coff[b + 1] - coff[b], [&](int64_t i) { return __dmul_rn(zb[i], zb[i]); },
+      [](double t, const double* term, int count) {
+#pragma unroll 16
+        for (int i = 0; i < count; ++i) t = __dadd_rn(t, term[i]);
+        return t;
+      });
+  if (threadIdx.x != 0) return;
   const double nz = __dsqrt_rn(acc);
   nz_out[b] = nz;
   if (nz == 0.0) {
@@ -675,12 +684,11 @@ struct MultiEngine {
     double* d_nz = dalloc<double>(K);
     double* d_s = dalloc<double>(K);
     int32_t* d_pdone = dalloc<int32_t>(K);
-    const unsigned kb = static_cast<unsigned>((K + kBlock - 1) / kBlock);
     k_pi_init<<<blocks(std::max<int64_t>(N, K)), kBlock, 0, stream>>>(N, K, d_cinst, d_co, d_nnz, dx, d_pdone, d_s);
     for (int it = 0; it < iters; ++it) {
       k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), dx, dy);
       k_spmv<<<blocks(N), kBlock, 0, stream>>>(N, 1, viewAT(), dy, dz);
-      k_pi_norm<<<kb, kBlock, 0, stream>>>(K, d_co, dz, d_pdone, d_nz, d_s);
+      k_pi_norm<<<K, kOrderedThreads, 0, stream>>>(d_co, dz, d_pdone, d_nz, d_s);
       k_pi_scale<<<blocks(N), kBlock, 0, stream>>>(N, d_cinst, d_pdone, d_nz, dz, dx);
     }
     B2P_CUDA(cudaGetLastError());
