@@ -24,9 +24,10 @@
 // strides, so either operand may be used transposed.  Waits are bounded: on
 // a timeout the kernel records an error, frees its TMEM and returns.
 //
-// When both operands are K-contiguous, the TMA form at the end of this file
-// (k_gemm_bf16_tma) replaces the threads' copies with tensor-map copies into
-// 128-byte-swizzled stages and splits the CTA into producer and MMA warps.
+// When each operand has a contiguous dimension and 16-byte aligned rows, the
+// TMA form at the end of this file (k_gemm_group) replaces the threads' copies
+// with tensor-map copies into 128-byte-swizzled stages and splits the CTA into
+// producer and MMA warps; the form here runs what is left (other strides).
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (the type only; maps are encoded through the runtime's driver entry point)
@@ -158,64 +159,124 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
   return false;
 }
 
-// Epilogue of one 128 x BN tile: thread = tile row (TMEM lane), 8 columns
-// per tcgen05.ld; alpha, bias, ReLU and the 0/1 mask applied in FP32; a
-// thread's 8 consecutive outputs go out as 16- or 32-byte vector stores when
-// the row stride and base allow it (one sector per store instead of eight
-// scattered ones).
+// Epilogue of one 128 x BN tile, 32 columns at a time: tcgen05.ld gives a
+// thread one tile row (TMEM lane), which goes through the warp's 4 KB of
+// `stage` (16-byte chunks XOR-swizzled by row, conflict-free both ways) to
+// come back as four columns of eight rows, so that the bias is loaded once,
+// and mask and outputs move as whole row segments (128 bytes of FP32); alpha,
+// bias, ReLU and the 0/1 mask are applied in FP32.  Written from the row
+// layout with every option tested per column, this took 228 cycles a column:
+// 14,600 of the 21,600 cycles of a 512 x 512 x 512 product in 128 x 64 tiles
+// (B2P_EPI here).
 template <int BN>
-__device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, uint32_t tmem, int m0, int n0, int warp, int lane) {
-  constexpr int kGemmBN = BN;
-  const int row = warp * 32 + lane;
-  const int gm = m0 + row;
-  const bool vec_f = g.cf && g.ldcf % 4 == 0 && (reinterpret_cast<uintptr_t>(g.cf) & 15) == 0;
-  const bool vec_b = g.cb && g.ldcb % 8 == 0 && (reinterpret_cast<uintptr_t>(g.cb) & 15) == 0;
-  for (int c = 0; c < kGemmBN; c += 8) {
-    uint32_t r[8];
-    const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c);
+__device__ __forceinline__ void gemm_epilogue(const GemmArgs& ga, uint32_t tmem, int m0, int n0, unsigned char* stage) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int M = ga.M, N = ga.N, relu = ga.relu;
+  const float alpha = ga.alpha;
+  const float* __restrict__ bias = ga.bias;
+  const __nv_bfloat16* __restrict__ mask = ga.mask;
+  float* __restrict__ cf = ga.cf;
+  __nv_bfloat16* __restrict__ cb = ga.cb;
+  const int64_t ldm = ga.ldm, ldcf = ga.ldcf, ldcb = ga.ldcb;
+  const auto aligned = [](const void* p, int bytes, int64_t ld) {
+    return ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0;
+  };
+  const bool vec = (!cf || aligned(cf, 16, ldcf)) && (!cb || aligned(cb, 8, ldcb)) && (!mask || aligned(mask, 8, ldm));
+  const bool rows_in = vec && m0 + kGemmBM <= M;
+  float4* tile = reinterpret_cast<float4*>(stage) + warp * 256;  // 32 rows x 8 chunks of 4 columns
+  const int quad = lane & 7, sub = lane >> 3;
+  for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 32) {
+    uint32_t r[32];
+    const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0);
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    if (gm >= g.M || n0 + c >= g.N) continue;
-    float v[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int gn = n0 + c + q;
-      float t = __uint_as_float(r[q]) * g.alpha;
-      if (gn < g.N) {
-        if (g.bias) t += g.bias[gn];
-        if (g.relu) t = t > 0.0f ? t : 0.0f;
-        if (g.mask && !(__bfloat162float(g.mask[gm * g.ldm + gn]) > 0.0f)) t = 0.0f;
+    for (int q = 0; q < 8; ++q)
+      tile[lane * 8 + (q ^ (lane & 7))] =
+          make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
+                      __uint_as_float(r[4 * q + 3]));
+    __syncwarp();
+    const int gn = n0 + c0 + 4 * quad, gm0 = m0 + warp * 32 + sub;
+    if (rows_in && n0 + c0 + 32 <= N) {
+      // straight-line: each option is one branch around 32 independent
+      // operations (a warp per scheduler has only its own parallelism to
+      // hide latencies with)
+      float4 v[8];
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int row = it * 4 + sub;
+        v[it] = tile[row * 8 + (quad ^ (row & 7))];
       }
-      v[q] = t;
-    }
-    const bool full = n0 + c + 8 <= g.N;
-    if (g.cf) {
-      float* dst = g.cf + gm * g.ldcf + n0 + c;
-      if (vec_f && full) {
-        reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-      } else {
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (n0 + c + q < g.N) dst[q] = v[q];
+      for (int it = 0; it < 8; ++it)
+        v[it] = make_float4(v[it].x * alpha, v[it].y * alpha, v[it].z * alpha, v[it].w * alpha);
+      if (bias) {
+        const float b0 = bias[gn], b1 = bias[gn + 1], b2 = bias[gn + 2], b3 = bias[gn + 3];
+#pragma unroll
+        for (int it = 0; it < 8; ++it)
+          v[it] = make_float4(v[it].x + b0, v[it].y + b1, v[it].z + b2, v[it].w + b3);
+      }
+      if (relu) {
+#pragma unroll
+        for (int it = 0; it < 8; ++it)
+          v[it] = make_float4(v[it].x > 0.0f ? v[it].x : 0.0f, v[it].y > 0.0f ? v[it].y : 0.0f,
+                              v[it].z > 0.0f ? v[it].z : 0.0f, v[it].w > 0.0f ? v[it].w : 0.0f);
+      }
+      if (mask) {
+        const __nv_bfloat16* src = mask + gm0 * ldm + gn;
+        uint2 w[8];
+#pragma unroll
+        for (int it = 0; it < 8; ++it) w[it] = *reinterpret_cast<const uint2*>(src + it * 4 * ldm);
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const __nv_bfloat162 w0 = *reinterpret_cast<const __nv_bfloat162*>(&w[it].x);
+          const __nv_bfloat162 w1 = *reinterpret_cast<const __nv_bfloat162*>(&w[it].y);
+          v[it] = make_float4(__low2float(w0) > 0.0f ? v[it].x : 0.0f, __high2float(w0) > 0.0f ? v[it].y : 0.0f,
+                              __low2float(w1) > 0.0f ? v[it].z : 0.0f, __high2float(w1) > 0.0f ? v[it].w : 0.0f);
+        }
+      }
+      if (cf) {
+        float* dst = cf + gm0 * ldcf + gn;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) *reinterpret_cast<float4*>(dst + it * 4 * ldcf) = v[it];
+      }
+      if (cb) {
+        __nv_bfloat16* dst = cb + gm0 * ldcb + gn;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[it].x, v[it].y), h1 = __floats2bfloat162_rn(v[it].z, v[it].w);
+          uint2 h;
+          h.x = *reinterpret_cast<const uint32_t*>(&h0);
+          h.y = *reinterpret_cast<const uint32_t*>(&h1);
+          *reinterpret_cast<uint2*>(dst + it * 4 * ldcb) = h;
+        }
+      }
+    } else {
+      for (int it = 0; it < 8; ++it) {
+        const int row = it * 4 + sub, gm = gm0 + it * 4;
+        const float4 t = tile[row * 8 + (quad ^ (row & 7))];
+        const float v[4] = {t.x, t.y, t.z, t.w};
+        if (gm >= M) break;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (gn + q >= N) break;
+          float o = v[q] * alpha;
+          if (bias) o += bias[gn + q];
+          if (relu) o = o > 0.0f ? o : 0.0f;
+          if (mask && !(__bfloat162float(mask[gm * ldm + gn + q]) > 0.0f)) o = 0.0f;
+          if (cf) cf[gm * ldcf + gn + q] = o;
+          if (cb) cb[gm * ldcb + gn + q] = __float2bfloat16(o);
+        }
       }
     }
-    if (g.cb) {
-      __nv_bfloat16* dst = g.cb + gm * g.ldcb + n0 + c;
-      if (vec_b && full) {
-        __align__(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) h[q] = __float2bfloat16(v[q]);
-        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (n0 + c + q < g.N) dst[q] = __float2bfloat16(v[q]);
-      }
-    }
+    __syncwarp();
   }
 }
 
@@ -229,7 +290,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tc(GemmArgs g) {
   __shared__ __align__(8) uint64_t mbar[kGemmStages];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int failed_sh;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5;
   const int m0 = blockIdx.x * kGemmBM, n0 = blockIdx.y * kGemmBN;
 
   if (tid == 0) {
@@ -314,7 +375,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tc(GemmArgs g) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!failed_sh) {
-    gemm_epilogue<kGemmBN>(g, tmem, m0, n0, warp, lane);
+    gemm_epilogue<kGemmBN>(g, tmem, m0, n0, smem);
   } else if (tid == 0) {
     atomicExch(g.error, 1);
   }
@@ -326,42 +387,99 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tc(GemmArgs g) {
 
 
 // ---------------------------------------------------------------------------
-// TMA form, for operands whose K dimension is contiguous (A row-major M x K,
-// B stored N x K) with 16-byte aligned rows.  The same 128 x BN tiles and
-// stage counts, but the operands are brought in by the tensor memory
-// accelerator (cp.async.bulk.tensor.2d, one 64 x rows box per operand and
-// chunk, zero-filled past the edges) into the 128-byte-swizzled K-major
-// layout, and the CTA's roles are split: warp 0 issues the copies, warp 1
-// the MMAs (one lane each, the other lanes following in step so that no lane
-// spins beside them), and all four warps run the epilogue.  Each stage
-// has a "full" mbarrier (the copies' bytes arrived) and an "empty" one (the
-// MMAs that read it completed); the producer refills a stage once it is
-// empty, so up to S chunks are in flight while the tensor core works.  Every
-// wait is bounded: on a timeout the kernel records an error, waits (bounded)
-// for the copies it issued, frees its TMEM and returns.
+// TMA form, for operands with one contiguous dimension -- K (A row-major
+// M x K, B stored N x K) or the other one (A stored K x M, B stored K x N) --
+// and 16-byte aligned rows.  128 x BN tiles, brought in by the tensor memory
+// accelerator (cp.async.bulk.tensor.2d, zero-filled past the edges) into
+// 128-byte-swizzled stages, K-major (one 64 x rows box an operand and chunk)
+// or MN-major (one box of 64 x 64 for every 64 rows of the tile).  The CTA's
+// roles are split: warp 0 issues the copies, warp 1 the MMAs (one lane each,
+// the other lanes following in step so that no lane spins beside them), and
+// all four warps run the epilogue.  Each stage has a "full" mbarrier (the
+// copies' bytes arrived) and an "empty" one (the MMAs that read it
+// completed); the producer refills a stage once it is empty, so all stages
+// are in flight while the tensor core works.  Every wait is bounded: on a
+// timeout the kernel records an error, waits (bounded) for the copies it
+// issued, frees its TMEM and returns.
+//
+// One launch runs a group of up to two independent products and the two
+// small reductions that go with a layer's backward pass (the bias gradient's
+// column sums, the loss), each on blocks of its own: a 512 x 512 x 512
+// product alone is 32 tiles, a fifth of the SMs, and mostly launch and
+// pipeline latency.  Launches overlap their set-up with the previous
+// kernel's tail (programmatic dependent launch).
+//
+// Measured on the network's training step (batch 512, 512-wide layers; the
+// backward products' operands are not K-contiguous): 765 us a step in
+// element-copied stages with separate reductions, B2P_STEP_US here.
 
+// Most stages of a tile shape (the launch takes fewer where K is shorter, or
+// where two CTAs are to share an SM).
 template <int BN>
 struct GemmTmaTile {
-  static constexpr int kStages = BN == 256 ? 4 : 3;
   static constexpr int kABytes = kGemmBM * kGemmBK * 2;  // 16 KB
   static constexpr int kBBytes = BN * kGemmBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kMaxStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int kSharedStages = BN == 256 ? 4 : BN == 128 ? 3 : 4;  // two CTAs per SM up to BN = 128
   // + 1 KB so that the stages can start on a 1,024-byte boundary (the
   // period of the 128-byte swizzle)
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+  __host__ __device__ static constexpr int smem_bytes(int stages) { return stages * kStageBytes + 1024; }
+};
+constexpr int kGemmMaxStages = 8;
+
+struct GemmProblem {
+  alignas(64) CUtensorMap a;
+  alignas(64) CUtensorMap b;
+  GemmArgs g;
+  int32_t first, blocks;  // its blocks of the grid
+  int32_t tiles_m;
+  int32_t a_mn, b_mn;  // the operand's contiguous dimension is M / N, not K
 };
 
-// UMMA shared-memory descriptor, K-major, 128-byte swizzle: rows of 64 BF16
+// out[c] = sum_r x[r * cols + c], rows in order.
+struct GroupColsum {
+  const float* x;
+  float* out;
+  int32_t rows, cols;
+  int32_t first, blocks;
+};
+
+// *loss = 0.5 * sum(partial) * inv_rows (in order), *accum += that * weight.
+struct GroupLoss {
+  const double* partial;
+  double* loss;
+  double* accum;
+  double inv_rows, weight;
+  int32_t count;
+  int32_t first, blocks;
+};
+
+struct GemmGroup {
+  GemmProblem p[2];
+  GroupColsum colsum;
+  GroupLoss loss;
+  int32_t problems;
+  int32_t stages;
+};
+
+__device__ __forceinline__ void gemm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void gemm_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" :::); }
+
+// UMMA shared-memory descriptor, 128-byte swizzle.  K-major: rows of 64 BF16
 // (128 bytes) as the copies wrote them, 8-row groups SBO = 1,024 bytes apart,
-// LBO unused (1).  addr advances by 32 bytes per K = 16 step inside the
-// 128-byte row; the swizzle is applied to the absolute address bits.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
+// LBO unused (1); the address advances by 32 bytes per K = 16 step inside the
+// 128-byte row.  MN-major: K rows of 64 M / N elements (128 bytes), groups of
+// 8 K rows SBO = 1,024 bytes apart, blocks of 64 M / N elements LBO = 64 x 128
+// bytes apart; the address advances by 16 rows per K = 16 step.  The swizzle
+// is applied to the absolute address bits.
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr, int mn) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((addr >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>(1) << 16;            // LBO (unused for swizzled K-major)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;    // SBO
-  d |= static_cast<uint64_t>(1) << 46;            // descriptor version (Blackwell)
-  d |= static_cast<uint64_t>(2) << 61;            // layout type SWIZZLE_128B
+  d |= static_cast<uint64_t>(mn ? (kGemmBK * 128) >> 4 : 1) << 16;  // LBO
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;                      // SBO
+  d |= static_cast<uint64_t>(1) << 46;                              // descriptor version (Blackwell)
+  d |= static_cast<uint64_t>(2) << 61;                              // layout type SWIZZLE_128B
   return d;
 }
 
@@ -373,18 +491,78 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// One operand's rows [r0, r0 + rows) x K columns [k0, k0 + 64) of a chunk.
+__device__ __forceinline__ void tma_load_operand(uint32_t dst, const CUtensorMap* map, int mn, int rows, int r0, int k0,
+                                                 uint32_t bar) {
+  if (!mn) {
+    tma_load_2d(dst, map, k0, r0, bar);
+  } else {
+    for (int q = 0; q < rows; q += 64) tma_load_2d(dst + q * kGemmBK * 2, map, r0 + q, k0, bar);
+  }
+}
+
+// Column sums of 32 columns: the rows staged in shared memory (up to `room`
+// at a time, all their loads in flight), one thread per column adding them
+// in order.
+__device__ __forceinline__ void group_colsum(const GroupColsum& j, float* stage, int room) {
+  const int c0 = (blockIdx.x - j.first) * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = c0 + lane;
+  float s = 0.0f;
+  for (int r0 = 0; r0 < j.rows; r0 += room) {
+    const int cnt = j.rows - r0 < room ? j.rows - r0 : room;
+    if (c < j.cols) {
+#pragma unroll 16
+      for (int r = warp; r < cnt; r += kGemmThreads / 32)
+        stage[r * 32 + lane] = __ldcg(j.x + static_cast<int64_t>(r0 + r) * j.cols + c);
+    }
+    __syncthreads();
+    if (warp == 0 && c < j.cols) {
+#pragma unroll 16
+      for (int r = 0; r < cnt; ++r) s += stage[r * 32 + lane];
+    }
+    __syncthreads();
+  }
+  if (warp == 0 && c < j.cols) j.out[c] = s;
+}
+
+__device__ __forceinline__ void group_loss(const GroupLoss& j, double* stage) {
+  for (int i = threadIdx.x; i < j.count; i += kGemmThreads) stage[i] = __ldcg(j.partial + i);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double s = 0.0;
+#pragma unroll 8
+  for (int i = 0; i < j.count; ++i) s += stage[i];
+  const double l = 0.5 * s * j.inv_rows;
+  if (j.loss) *j.loss = l;
+  if (j.accum) *j.accum += l * j.weight;
+}
+
 template <int BN>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_constant__ CUtensorMap map_a,
-                                                                 const __grid_constant__ CUtensorMap map_b,
-                                                                 GemmArgs g) {
+__global__ void __launch_bounds__(kGemmThreads) k_gemm_group(const __grid_constant__ GemmGroup G) {
   using Tile = GemmTmaTile<BN>;
-  constexpr int S = Tile::kStages;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full[S], empty[S], done;
+  __shared__ __align__(8) uint64_t full[kGemmMaxStages], empty[kGemmMaxStages], done;
   __shared__ uint32_t tmem_base_sh;
   __shared__ int failed_sh, issued_sh, consumed_sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * kGemmBM, n0 = blockIdx.y * BN;
+  const int blk = blockIdx.x;
+  if (blk >= G.loss.first && blk < G.loss.first + G.loss.blocks) {
+    gemm_pdl_wait();
+    gemm_pdl_launch();
+    group_loss(G.loss, reinterpret_cast<double*>(smem_raw));
+    return;
+  }
+  if (blk >= G.colsum.first && blk < G.colsum.first + G.colsum.blocks) {
+    gemm_pdl_wait();
+    gemm_pdl_launch();
+    group_colsum(G.colsum, reinterpret_cast<float*>(smem_raw), Tile::smem_bytes(G.stages) / 128);
+    return;
+  }
+  const GemmProblem& P = G.p[G.problems > 1 && blk >= G.p[1].first ? 1 : 0];
+  const GemmArgs& g = P.g;
+  const int S = G.stages;
+  const int tile = blk - P.first;
+  const int m0 = tile % P.tiles_m * kGemmBM, n0 = tile / P.tiles_m * BN;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // stage 0, 1,024-byte aligned
   const int nchunks = (g.K + kGemmBK - 1) / kGemmBK;
@@ -399,6 +577,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
     failed_sh = 0;
     issued_sh = 0;
     consumed_sh = 0;
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&P.a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&P.b)) : "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
@@ -410,19 +590,19 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_sh;
+  // everything above is this CTA's own; the operands, and what the outputs
+  // overwrite, belong to the kernels before
+  gemm_pdl_wait();
+  gemm_pdl_launch();
 
   if (warp == 0) {
     // producer warp (lane 0 issues): chunk ch into stage ch % S once the MMAs
     // of chunk ch - S are done
-    if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
-    }
-    int ch = 0;
+    int ch = 0, st = 0;
+    uint32_t round = 0;
     for (; ch < nchunks; ++ch) {
-      const int st = ch % S;
       bool ok = true;
-      if (ch >= S) ok = mbar_wait(smem_u32(&empty[st]), static_cast<uint32_t>((ch / S - 1) & 1));
+      if (round > 0) ok = mbar_wait(smem_u32(&empty[st]), (round - 1) & 1);
       if (!__all_sync(0xffffffffu, ok) || *reinterpret_cast<volatile int*>(&failed_sh)) {
         if (lane == 0) failed_sh = 1;
         break;
@@ -432,20 +612,22 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[st])),
                      "r"(Tile::kStageBytes)
                      : "memory");
-        tma_load_2d(sa, &map_a, ch * kGemmBK, m0, smem_u32(&full[st]));
-        tma_load_2d(sb, &map_b, ch * kGemmBK, n0, smem_u32(&full[st]));
+        tma_load_operand(sa, &P.a, P.a_mn, kGemmBM, m0, ch * kGemmBK, smem_u32(&full[st]));
+        tma_load_operand(sb, &P.b, P.b_mn, BN, n0, ch * kGemmBK, smem_u32(&full[st]));
       }
       __syncwarp();
+      if (++st == S) st = 0, ++round;
     }
     if (lane == 0) issued_sh = ch;
   } else if (warp == 1) {
     // MMA warp (lane 0 issues): four K = 16 steps per chunk, then commit the
     // stage back
-    const uint32_t idesc = umma_idesc_bf16(BN);
-    int ch = 0;
+    const uint32_t idesc = umma_idesc_bf16(BN) | (P.a_mn ? 1u << 15 : 0u) | (P.b_mn ? 1u << 16 : 0u);
+    const uint32_t step_a = P.a_mn ? 16 * 128 : 32, step_b = P.b_mn ? 16 * 128 : 32;
+    int ch = 0, st = 0;
+    uint32_t round = 0;
     for (; ch < nchunks; ++ch) {
-      const int st = ch % S;
-      const bool ok = mbar_wait(smem_u32(&full[st]), static_cast<uint32_t>((ch / S) & 1));
+      const bool ok = mbar_wait(smem_u32(&full[st]), round & 1);
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) failed_sh = 1;
         break;
@@ -455,7 +637,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
         const uint32_t sa = base + st * Tile::kStageBytes, sb = sa + Tile::kABytes;
 #pragma unroll
         for (int s = 0; s < kGemmBK / 16; ++s) {
-          const uint64_t da = umma_desc_sw128(sa + s * 32), db = umma_desc_sw128(sb + s * 32);
+          const uint64_t da = umma_desc_sw128(sa + s * step_a, P.a_mn), db = umma_desc_sw128(sb + s * step_b, P.b_mn);
           const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
           asm volatile(
               "{\n\t.reg .pred p;\n\t"
@@ -470,6 +652,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
                      : "memory");
       }
       __syncwarp();
+      if (++st == S) st = 0, ++round;
     }
     if (lane == 0) {
       consumed_sh = ch;
@@ -485,7 +668,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tma(const __grid_con
   __syncwarp();  // the producer and MMA lanes rejoin their warps before tcgen05.ld
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!failed_sh) {
-    gemm_epilogue<BN>(g, tmem, m0, n0, warp, lane);
+    gemm_epilogue<BN>(g, tmem, m0, n0, smem_raw + (base - raw));
   } else if (tid == 0) {
     atomicExch(g.error, 1);
     // copies issued but not consumed still write into shared memory: wait for them

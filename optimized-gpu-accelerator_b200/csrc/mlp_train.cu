@@ -30,6 +30,8 @@ inline int ew_blocks(int64_t n) { return static_cast<int>(std::max<int64_t>(1, s
 __global__ void k_gather(int32_t rows, int32_t din, int32_t dout, const float* __restrict__ x,
                          const float* __restrict__ y, const int32_t* __restrict__ perm, int64_t offset,
                          __nv_bfloat16* __restrict__ xb, float* __restrict__ yt) {
+  gemm_pdl_wait();
+  gemm_pdl_launch();
   const int64_t nin = static_cast<int64_t>(rows) * din, nout = static_cast<int64_t>(rows) * dout;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < nin + nout;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -49,6 +51,8 @@ __global__ void k_gather(int32_t rows, int32_t din, int32_t dout, const float* _
 __global__ void __launch_bounds__(kEw) k_mse_grad(int64_t count, float inv_rows, const float* __restrict__ out,
                                                   const float* __restrict__ target, float* __restrict__ gf,
                                                   __nv_bfloat16* __restrict__ gb, double* __restrict__ partial) {
+  gemm_pdl_wait();
+  gemm_pdl_launch();
   double s = 0.0;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(kEw) + threadIdx.x; e < count;
        e += static_cast<int64_t>(gridDim.x) * kEw) {
@@ -68,32 +72,13 @@ __global__ void __launch_bounds__(kEw) k_mse_grad(int64_t count, float inv_rows,
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
-// loss = 0.5 * sum(partials) / rows; stored to *loss and added, times
-// `weight`, to *accum (the epoch mean)
-__global__ void k_loss_finish(int32_t nblocks, const double* __restrict__ partial, double inv_rows, double* loss,
-                              double* accum, double weight) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < nblocks; ++i) s += partial[i];
-  const double l = 0.5 * s * inv_rows;
-  if (loss) *loss = l;
-  if (accum) *accum += l * weight;
-}
-
-// bias gradient: db[c] = sum_r G[r, c] (rows summed in order)
-__global__ void k_colsum(int32_t rows, int32_t cols, const float* __restrict__ g, float* __restrict__ db) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.0f;
-  for (int r = 0; r < rows; ++r) s += g[static_cast<int64_t>(r) * cols + c];
-  db[c] = s;
-}
-
 // Adam (decoupled weight decay on the entries flagged in `decay`), then the
 // BF16 copy of the parameters
 __global__ void k_adam(int64_t n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, const uint8_t* __restrict__ decay, float lr, float b1, float b2,
                        float c1, float c2, float eps, float wd, __nv_bfloat16* __restrict__ pb) {
+  gemm_pdl_wait();
+  gemm_pdl_launch();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float gi = g[i];
@@ -132,28 +117,34 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// Tensor map of a K-contiguous operand X(r, k) = X[r * sr + k], r < R,
-// k < K: 64 x box_rows boxes, 128-byte swizzle, zeros past the edges.
-bool encode_operand(CUtensorMap* map, const __nv_bfloat16* X, int64_t sr, int R, int K, int box_rows) {
+// How the TMA form reads an operand X(r, k) = X[r * sr + k * sk], r < R,
+// k < K: 0 = K-major, 1 = MN-major, -1 = not at all (a tensor map wants one
+// contiguous dimension and rows of a multiple of 16 bytes on a 16-byte
+// aligned base).
+int operand_major(const void* X, int64_t sr, int64_t sk, int R, int K) {
+  const auto rows_ok = [&](int64_t stride, int64_t inner) {
+    return stride >= inner && stride % 8 == 0 && stride < (int64_t{1} << 38);
+  };
+  if (K <= 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0) return -1;
+  if (sk == 1 && rows_ok(sr, K)) return 0;
+  if (sr == 1 && rows_ok(sk, R)) return 1;
+  return -1;
+}
+
+// Tensor map of such an operand, zeros past the edges, 128-byte swizzle:
+// boxes of 64 K columns x box_rows rows (K-major) or 64 rows x 64 K columns
+// (MN-major).
+bool encode_operand(CUtensorMap* map, const __nv_bfloat16* X, int64_t sr, int64_t sk, int R, int K, int mn,
+                    int box_rows) {
   const auto fn = tensor_map_encoder();
   if (!fn) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(R)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(sr) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kGemmBK), static_cast<cuuint32_t>(box_rows)};
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(mn ? R : K), static_cast<cuuint64_t>(mn ? K : R)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(mn ? sk : sr) * 2};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(mn ? kGemmBK : box_rows)};
   const cuuint32_t elem[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(X), dims, strides, box, elem,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The TMA form applies when both operands are K-contiguous with rows of a
-// multiple of 16 bytes on a 16-byte aligned base (the tensor map's rules).
-bool gemm_tma_ok(const GemmArgs& g) {
-  auto ok = [&](const void* X, int64_t sr, int64_t sk) {
-    return sk == 1 && sr >= g.K && sr % 8 == 0 && sr < (int64_t{1} << 38) &&
-           (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  };
-  return g.K > 0 && ok(g.A, g.sam, g.sak) && ok(g.B, g.sbn, g.sbk);
 }
 
 void set_gemm_attributes() {
@@ -167,42 +158,60 @@ void set_gemm_attributes() {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(k_gemm_bf16_tc<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  GemmTile<256>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_gemm_bf16_tma<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 GemmTmaTile<128>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_gemm_bf16_tma<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 GemmTmaTile<256>::kSmemBytes);
+    const auto group = [&](auto* fn, int bytes) {
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    group(k_gemm_group<64>, GemmTmaTile<64>::smem_bytes(GemmTmaTile<64>::kMaxStages));
+    group(k_gemm_group<128>, GemmTmaTile<128>::smem_bytes(GemmTmaTile<128>::kMaxStages));
+    group(k_gemm_group<256>, GemmTmaTile<256>::smem_bytes(GemmTmaTile<256>::kMaxStages));
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&gemm_sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
   });
   B2P_CUDA(err);
 }
 
-// 128 x 256 tiles when they still give every SM a CTA, else 128 x 128
-// (the network's small GEMMs need the wider grid); the TMA form when both
-// operands are K-contiguous, the cp.async form otherwise.
-void launch_gemm(const GemmArgs& g, cudaStream_t stream) {
-  if (g.M <= 0 || g.N <= 0) return;
-  int dev = 0;
-  B2P_CUDA(cudaGetDevice(&dev));
-  const int64_t mt = (g.M + kGemmBM - 1) / kGemmBM;
-  const int sms = gemm_sms[dev & 63];
-  const bool wide = sms > 0 && mt * ((g.N + 255) / 256) >= sms;
-  if (sms > 0 && gemm_tma_ok(g)) {
-    CUtensorMap ma, mb;
-    if (encode_operand(&ma, g.A, g.sam, g.M, g.K, kGemmBM) && encode_operand(&mb, g.B, g.sbn, g.N, g.K, wide ? 256 : 128)) {
-      if (wide) {
-        const dim3 grid(static_cast<unsigned>(mt), (g.N + 255) / 256);
-        k_gemm_bf16_tma<256><<<grid, kGemmThreads, GemmTmaTile<256>::kSmemBytes, stream>>>(ma, mb, g);
-      } else {
-        const dim3 grid(static_cast<unsigned>(mt), (g.N + 127) / 128);
-        k_gemm_bf16_tma<128><<<grid, kGemmThreads, GemmTmaTile<128>::kSmemBytes, stream>>>(ma, mb, g);
-      }
-      B2P_CUDA(cudaGetLastError());
-      return;
-    }
+// Launch with programmatic dependent launch (the kernel waits for the one
+// before it itself).
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  B2P_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+
+template <int BN>
+void launch_group_bn(GemmGroup& gr, cudaStream_t stream, int sms) {
+  using Tile = GemmTmaTile<BN>;
+  int next = 0, chunks = 2;
+  for (int i = 0; i < gr.problems; ++i) {
+    GemmProblem& p = gr.p[i];
+    p.tiles_m = (p.g.M + kGemmBM - 1) / kGemmBM;
+    p.first = next;
+    p.blocks = p.tiles_m * ((p.g.N + BN - 1) / BN);
+    next += p.blocks;
+    chunks = std::max(chunks, (p.g.K + kGemmBK - 1) / kGemmBK);
   }
-  if (wide) {
+  gr.colsum.first = next;
+  next += gr.colsum.blocks;
+  gr.loss.first = next;
+  next += gr.loss.blocks;
+  // one CTA per SM has the whole shared memory for its stages
+  gr.stages = std::min(chunks, next <= sms ? Tile::kMaxStages : Tile::kSharedStages);
+  if (next > 0)
+    launch_pdl(k_gemm_group<BN>, static_cast<unsigned>(next), kGemmThreads, Tile::smem_bytes(gr.stages), stream, gr);
+}
+
+void launch_gemm_strided(const GemmArgs& g, cudaStream_t stream, int sms) {
+  const int64_t mt = (g.M + kGemmBM - 1) / kGemmBM;
+  if (mt * ((g.N + 255) / 256) >= sms) {
     const dim3 grid(static_cast<unsigned>(mt), (g.N + 255) / 256);
     k_gemm_bf16_tc<256><<<grid, kGemmThreads, GemmTile<256>::kSmemBytes, stream>>>(g);
   } else {
@@ -211,6 +220,49 @@ void launch_gemm(const GemmArgs& g, cudaStream_t stream) {
   }
   B2P_CUDA(cudaGetLastError());
 }
+
+// Up to two independent products and the reductions of `jobs` (its colsum and
+// loss; blocks 0 = none) in one launch.  The widest tiles that still give
+// every SM a CTA, else the narrowest (128 x 64: a product too small to fill
+// the GPU is bound by its pipeline's latency, which more and shorter tiles
+// share out: 512 x 512 x 512 B2P_T128 us in 16 tiles of 128 x 128, B2P_T64 us
+// in 32 of 128 x 64).  A product whose strides a tensor map cannot describe
+// runs the cp.async form by itself.
+void launch_group(const GemmArgs* g, int count, GemmGroup jobs, cudaStream_t stream) {
+  int dev = 0;
+  B2P_CUDA(cudaGetDevice(&dev));
+  const int sms = gemm_sms[dev & 63];
+  GemmGroup& gr = jobs;
+  gr.problems = 0;
+  int64_t tiles256 = 0, tiles128 = 0;
+  for (int i = 0; i < count; ++i) {
+    if (g[i].M <= 0 || g[i].N <= 0) continue;
+    const int64_t mt = (g[i].M + kGemmBM - 1) / kGemmBM;
+    tiles256 += mt * ((g[i].N + 255) / 256);
+    tiles128 += mt * ((g[i].N + 127) / 128);
+  }
+  const int bn = tiles256 >= sms ? 256 : tiles128 >= sms ? 128 : 64;
+  for (int i = 0; i < count; ++i) {
+    const GemmArgs& a = g[i];
+    if (a.M <= 0 || a.N <= 0) continue;
+    GemmProblem& p = gr.p[gr.problems];
+    const int ma = operand_major(a.A, a.sam, a.sak, a.M, a.K), mb = operand_major(a.B, a.sbn, a.sbk, a.N, a.K);
+    if (ma >= 0 && mb >= 0 && encode_operand(&p.a, a.A, a.sam, a.sak, a.M, a.K, ma, kGemmBM) &&
+        encode_operand(&p.b, a.B, a.sbn, a.sbk, a.N, a.K, mb, bn)) {
+      p.g = a;
+      p.a_mn = ma;
+      p.b_mn = mb;
+      ++gr.problems;
+    } else {
+      launch_gemm_strided(a, stream, sms);
+    }
+  }
+  if (bn == 256) launch_group_bn<256>(gr, stream, sms);
+  else if (bn == 128) launch_group_bn<128>(gr, stream, sms);
+  else launch_group_bn<64>(gr, stream, sms);
+}
+
+void launch_gemm(const GemmArgs& g, cudaStream_t stream) { launch_group(&g, 1, GemmGroup{}, stream); }
 
 template <class T>
 T* dalloc(size_t count) {
@@ -346,32 +398,15 @@ struct Mlp {
   void loss_backward(int32_t rows, double* accum, double weight) {
     const int64_t cnt = static_cast<int64_t>(rows) * w[L];
     const int nb = static_cast<int>(std::min<int64_t>(kLossBlocks, (cnt + kEw - 1) / kEw));
-    k_mse_grad<<<nb, kEw, 0, stream>>>(cnt, 1.0f / static_cast<float>(rows), out, target, gf[0], gb[0], partial);
-    B2P_CUDA(cudaGetLastError());
-    k_loss_finish<<<1, 32, 0, stream>>>(nb, partial, 1.0 / rows, d_loss, accum, weight);
-    B2P_CUDA(cudaGetLastError());
+    launch_pdl(k_mse_grad, nb, kEw, 0, stream, cnt, 1.0f / static_cast<float>(rows), out, target, gf[0], gb[0], partial);
     int cur = 0;
     for (int l = L - 1; l >= 0; --l) {
       const int32_t wo = w[l + 1], wi = w[l];
-      // dW_l = G^T h_l  (wo x wi, K = rows)
-      GemmArgs g = gemm_base();
-      g.M = wo;
-      g.N = wi;
-      g.K = rows;
-      g.A = gb[cur];
-      g.sam = 1;
-      g.sak = wo;
-      g.B = act[l];
-      g.sbk = wi;
-      g.sbn = 1;
-      g.cf = grads + woff[l];
-      g.ldcf = wi;
-      launch_gemm(g, stream);
-      k_colsum<<<(wo + kEw - 1) / kEw, kEw, 0, stream>>>(rows, wo, gf[cur], grads + boff[l]);
-      B2P_CUDA(cudaGetLastError());
+      GemmArgs g[2];
+      int count = 0;
       if (l > 0) {
         // G_{l-1} = (G W_l) masked by relu'(h_l)  (rows x wi, K = wo)
-        GemmArgs h = gemm_base();
+        GemmArgs& h = g[count++] = gemm_base();
         h.M = rows;
         h.N = wi;
         h.K = wo;
@@ -387,9 +422,26 @@ struct Mlp {
         h.ldcf = wi;
         h.cb = gb[cur ^ 1];
         h.ldcb = wi;
-        launch_gemm(h, stream);
-        cur ^= 1;
       }
+      // dW_l = G^T h_l  (wo x wi, K = rows)
+      GemmArgs& d = g[count++] = gemm_base();
+      d.M = wo;
+      d.N = wi;
+      d.K = rows;
+      d.A = gb[cur];
+      d.sam = 1;
+      d.sak = wo;
+      d.B = act[l];
+      d.sbk = wi;
+      d.sbn = 1;
+      d.cf = grads + woff[l];
+      d.ldcf = wi;
+      // the bias gradient, and, beside the last layer, the loss
+      GemmGroup jobs{};
+      jobs.colsum = GroupColsum{gf[cur], grads + boff[l], rows, wo, 0, (wo + 31) / 32};
+      if (l == L - 1) jobs.loss = GroupLoss{partial, d_loss, accum, 1.0 / rows, weight, nb, 0, 1};
+      launch_group(g, count, jobs, stream);
+      cur ^= 1;
     }
   }
 
@@ -442,9 +494,8 @@ struct Mlp {
   void forward_dev(const float* dx, int64_t batch, float* dy, cudaStream_t s) {
     for (int64_t r0 = 0; r0 < batch; r0 += max_batch) {
       const int32_t rows = static_cast<int32_t>(std::min<int64_t>(max_batch, batch - r0));
-      k_gather<<<ew_blocks(static_cast<int64_t>(rows) * w[0]), kEw, 0, s>>>(rows, w[0], w[L], dx, nullptr, nullptr,
-                                                                            r0, act[0], nullptr);
-      B2P_CUDA(cudaGetLastError());
+      launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(rows) * w[0]), kEw, 0, s, rows, w[0], w[L], dx, nullptr,
+                 nullptr, r0, act[0], nullptr);
       forward(rows, dy + r0 * w[L], s);
     }
   }
@@ -458,9 +509,8 @@ struct Mlp {
     try {
       B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * batch * w[0], cudaMemcpyHostToDevice, stream));
       B2P_CUDA(cudaMemcpyAsync(dy, y, sizeof(float) * batch * w[L], cudaMemcpyHostToDevice, stream));
-      k_gather<<<ew_blocks(static_cast<int64_t>(batch) * (w[0] + w[L])), kEw, 0, stream>>>(batch, w[0], w[L], dx, dy,
-                                                                                           nullptr, 0, act[0], target);
-      B2P_CUDA(cudaGetLastError());
+      launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(batch) * (w[0] + w[L])), kEw, 0, stream, batch, w[0], w[L],
+                 dx, dy, nullptr, 0, act[0], target);
       forward(batch, out, stream);
       d_loss = dl;
       loss_backward(batch, nullptr, 0.0);
@@ -514,9 +564,8 @@ struct Mlp {
         std::shuffle(perm.begin(), perm.end(), rng);
         B2P_CUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, stream));
         for (int64_t sidx = 0; sidx < steps_per_epoch; ++sidx, ++t) {
-          k_gather<<<ew_blocks(static_cast<int64_t>(bs) * (w[0] + w[L])), kEw, 0, stream>>>(
-              bs, w[0], w[L], dx, dy, dperm, sidx * bs, act[0], target);
-          B2P_CUDA(cudaGetLastError());
+          launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(bs) * (w[0] + w[L])), kEw, 0, stream, bs, w[0], w[L], dx,
+                     dy, dperm, sidx * bs, act[0], target);
           forward(bs, out, stream);
           loss_backward(bs, dl + 1 + ep, 1.0 / static_cast<double>(steps_per_epoch));
           ++step;
@@ -524,11 +573,9 @@ struct Mlp {
           const double lr = o.lr_final + 0.5 * (o.lr - o.lr_final) * (1.0 + std::cos(M_PI * frac));
           const double c1 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta1), static_cast<double>(step)));
           const double c2 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta2), static_cast<double>(step)));
-          k_adam<<<ew_blocks(nparams), kEw, 0, stream>>>(nparams, params, grads, adam_m, adam_v, decay,
-                                                         static_cast<float>(lr), o.beta1, o.beta2,
-                                                         static_cast<float>(c1), static_cast<float>(c2), o.eps,
-                                                         o.weight_decay, pbf);
-          B2P_CUDA(cudaGetLastError());
+          launch_pdl(k_adam, ew_blocks(nparams), kEw, 0, stream, nparams, params, grads, adam_m, adam_v, decay,
+                     static_cast<float>(lr), o.beta1, o.beta2, static_cast<float>(c1), static_cast<float>(c2), o.eps,
+                     o.weight_decay, pbf);
         }
       }
       std::vector<double> hl(1 + std::max(o.epochs, 1));
