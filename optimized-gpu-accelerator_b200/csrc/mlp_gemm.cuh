@@ -72,7 +72,7 @@ struct GemmArgs {
   int64_t ldcf;
   __nv_bfloat16* cb;  // BF16 output, or NULL
   int64_t ldcb;
-  int32_t* error;  // set to 1 on an mbarrier timeout
+  int32_t* error;  // set to 1 on an mbarrier timeout (page-locked host memory)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tc(GemmArgs g) {
   if (!failed_sh) {
     gemm_epilogue<kGemmBN>(g, tmem, m0, n0, smem);
   } else if (tid == 0) {
-    atomicExch(g.error, 1);
+    *const_cast<volatile int32_t*>(g.error) = 1;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_group(const __grid_consta
   if (!failed_sh) {
     gemm_epilogue<BN>(g, tmem, m0, n0, smem_raw + (base - raw));
   } else if (tid == 0) {
-    atomicExch(g.error, 1);
+    *const_cast<volatile int32_t*>(g.error) = 1;
     // copies issued but not consumed still write into shared memory: wait for them
     for (int ch = consumed_sh; ch < issued_sh; ++ch)
       mbar_wait(smem_u32(&full[ch % S]), static_cast<uint32_t>((ch / S) & 1));

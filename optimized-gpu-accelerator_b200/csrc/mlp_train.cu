@@ -279,6 +279,53 @@ void launch_group(const GemmArgs* g, int count, GemmGroup jobs, cudaStream_t str
 
 void launch_gemm(const GemmArgs& g, cudaStream_t stream) { launch_group(&g, 1, GemmGroup{}, stream); }
 
+// A page-locked word that a GEMM's timeout sets and the host reads once the
+// stream is synchronised: no memset before the call, no copy after it.
+class ErrorWord {
+ public:
+  ErrorWord() : word_(static_cast<volatile int32_t*>(PinnedCache::get(sizeof(int32_t)))) { *word_ = 0; }
+  ~ErrorWord() { PinnedCache::put(const_cast<int32_t*>(word_), sizeof(int32_t)); }
+  ErrorWord(const ErrorWord&) = delete;
+  ErrorWord& operator=(const ErrorWord&) = delete;
+  int32_t* device() const { return const_cast<int32_t*>(word_); }
+  // Waits for the stream; throws if a wait of its kernels timed out.
+  void check(cudaStream_t stream) {
+    B2P_CUDA(cudaStreamSynchronize(stream));
+    if (!*word_) return;
+    *word_ = 0;
+    throw Error(B2P_ERR_CUDA, "tensor-core GEMM: mbarrier wait timed out");
+  }
+
+ private:
+  volatile int32_t* word_;
+};
+
+// Buffers of one call on a stream, from the device's stream-ordered pool: a
+// cudaMalloc / cudaFree pair costs 30 us to milliseconds a call and waits for
+// the whole device.
+class CallBuffers {
+ public:
+  CallBuffers(int dev, cudaStream_t stream) : dev_(dev), stream_(stream) {}
+  ~CallBuffers() {
+    for (void* p : owned_) cudaFreeAsync(p, stream_);
+  }
+  CallBuffers(const CallBuffers&) = delete;
+  CallBuffers& operator=(const CallBuffers&) = delete;
+  template <class T>
+  T* get(size_t count) {
+    if (!count) return nullptr;
+    void* p = nullptr;
+    B2P_CUDA(cudaMallocFromPoolAsync(&p, count * sizeof(T), device_pool(dev_), stream_));
+    owned_.push_back(p);
+    return static_cast<T*>(p);
+  }
+
+ private:
+  int dev_;
+  cudaStream_t stream_;
+  std::vector<void*> owned_;
+};
+
 template <class T>
 T* dalloc(size_t count) {
   void* p = nullptr;
@@ -305,7 +352,7 @@ struct Mlp {
   __nv_bfloat16* gb[2] = {nullptr, nullptr};
   double* partial = nullptr;                  // kLossBlocks
   double* d_loss = nullptr;                   // [0] last loss, [1..] epoch sums
-  int32_t* d_error = nullptr;
+  ErrorWord error;
   std::vector<void*> owned;
 
   ~Mlp() {
@@ -363,8 +410,6 @@ struct Mlp {
       gb[i] = alloc<__nv_bfloat16>(static_cast<size_t>(mb) * wmax);
     }
     partial = alloc<double>(kLossBlocks);
-    d_error = alloc<int32_t>(1);
-    B2P_CUDA(cudaMemsetAsync(d_error, 0, sizeof(int32_t), stream));
     set_gemm_attributes();
     reset_moments();
     B2P_CUDA(cudaStreamSynchronize(stream));
@@ -379,7 +424,7 @@ struct Mlp {
   GemmArgs gemm_base() const {
     GemmArgs g{};
     g.alpha = 1.0f;
-    g.error = d_error;
+    g.error = error.device();
     return g;
   }
 
@@ -460,12 +505,7 @@ struct Mlp {
     }
   }
 
-  void check_error() {
-    int32_t h = 0;
-    B2P_CUDA(cudaMemcpyAsync(&h, d_error, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    B2P_CUDA(cudaStreamSynchronize(stream));
-    if (h) throw Error(B2P_ERR_CUDA, "tensor-core GEMM: mbarrier wait timed out");
-  }
+  void check_error() { error.check(stream); }
 
   void set_params(const float* hp) {
     B2P_CUDA(cudaSetDevice(device));
@@ -485,25 +525,16 @@ struct Mlp {
   void forward_host(const float* x, int64_t batch, float* y) {
     B2P_CUDA(cudaSetDevice(device));
     if (batch < 0) throw Error(B2P_ERR_INVALID, "negative batch");
-    float* dx = alloc_scratch_x(batch);
-    float* dy = dalloc<float>(static_cast<size_t>(batch) * w[L]);
-    try {
-      if (batch) {
-        B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * batch * w[0], cudaMemcpyHostToDevice, stream));
-        forward_dev(dx, batch, dy, stream);
-        B2P_CUDA(cudaMemcpyAsync(y, dy, sizeof(float) * batch * w[L], cudaMemcpyDeviceToHost, stream));
-      }
-      check_error();
-    } catch (...) {
-      cudaFree(dx);
-      cudaFree(dy);
-      throw;
+    CallBuffers buf(device, stream);
+    float* dx = buf.get<float>(static_cast<size_t>(batch) * w[0]);
+    float* dy = buf.get<float>(static_cast<size_t>(batch) * w[L]);
+    if (batch) {
+      B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * batch * w[0], cudaMemcpyHostToDevice, stream));
+      forward_dev(dx, batch, dy, stream);
+      B2P_CUDA(cudaMemcpyAsync(y, dy, sizeof(float) * batch * w[L], cudaMemcpyDeviceToHost, stream));
     }
-    cudaFree(dx);
-    cudaFree(dy);
+    check_error();
   }
-
-  float* alloc_scratch_x(int64_t batch) { return dalloc<float>(static_cast<size_t>(batch) * w[0]); }
 
   // chunks of max_batch rows through the activation buffers
   void forward_dev(const float* dx, int64_t batch, float* dy, cudaStream_t s) {
@@ -518,34 +549,29 @@ struct Mlp {
   void loss_grad(const float* x, const float* y, int32_t batch, double* loss, float* grad) {
     B2P_CUDA(cudaSetDevice(device));
     if (batch < 1 || batch > max_batch) throw Error(B2P_ERR_INVALID, "batch must be in [1, max_batch]");
-    float* dx = dalloc<float>(static_cast<size_t>(batch) * w[0]);
-    float* dy = dalloc<float>(static_cast<size_t>(batch) * w[L]);
-    double* dl = dalloc<double>(1);
-    try {
-      B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * batch * w[0], cudaMemcpyHostToDevice, stream));
-      B2P_CUDA(cudaMemcpyAsync(dy, y, sizeof(float) * batch * w[L], cudaMemcpyHostToDevice, stream));
-      launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(batch) * (w[0] + w[L])), kEw, 0, stream, batch, w[0], w[L],
-                 dx, dy, nullptr, 0, act[0], target);
-      forward(batch, out, stream);
-      d_loss = dl;
-      loss_backward(batch, nullptr, 0.0);
-      double hl = 0;
-      B2P_CUDA(cudaMemcpyAsync(&hl, dl, sizeof(double), cudaMemcpyDeviceToHost, stream));
-      if (grad) B2P_CUDA(cudaMemcpyAsync(grad, grads, sizeof(float) * nparams, cudaMemcpyDeviceToHost, stream));
-      check_error();
-      if (loss) *loss = hl;
-    } catch (...) {
-      cudaFree(dx);
-      cudaFree(dy);
-      cudaFree(dl);
-      d_loss = nullptr;
-      throw;
-    }
-    cudaFree(dx);
-    cudaFree(dy);
-    cudaFree(dl);
-    d_loss = nullptr;
+    CallBuffers buf(device, stream);
+    float* dx = buf.get<float>(static_cast<size_t>(batch) * w[0]);
+    float* dy = buf.get<float>(static_cast<size_t>(batch) * w[L]);
+    LossGuard guard{*this, buf.get<double>(1)};
+    B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * batch * w[0], cudaMemcpyHostToDevice, stream));
+    B2P_CUDA(cudaMemcpyAsync(dy, y, sizeof(float) * batch * w[L], cudaMemcpyHostToDevice, stream));
+    launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(batch) * (w[0] + w[L])), kEw, 0, stream, batch, w[0], w[L], dx,
+               dy, nullptr, 0, act[0], target);
+    forward(batch, out, stream);
+    loss_backward(batch, nullptr, 0.0);
+    double hl = 0;
+    B2P_CUDA(cudaMemcpyAsync(&hl, d_loss, sizeof(double), cudaMemcpyDeviceToHost, stream));
+    if (grad) B2P_CUDA(cudaMemcpyAsync(grad, grads, sizeof(float) * nparams, cudaMemcpyDeviceToHost, stream));
+    check_error();
+    if (loss) *loss = hl;
   }
+
+  // d_loss for the time of one call
+  struct LossGuard {
+    Mlp& net;
+    LossGuard(Mlp& n, double* p) : net(n) { net.d_loss = p; }
+    ~LossGuard() { net.d_loss = nullptr; }
+  };
 
   void train(const float* x, const float* y, int64_t count, const b2p_mlp_train_options& o, float* epoch_loss) {
     B2P_CUDA(cudaSetDevice(device));
@@ -555,56 +581,44 @@ struct Mlp {
     const int32_t bs = static_cast<int32_t>(std::min<int64_t>(o.batch, count));
     const int64_t steps_per_epoch = count / bs;
     const int64_t total = steps_per_epoch * o.epochs;
-    float* dx = dalloc<float>(static_cast<size_t>(count) * w[0]);
-    float* dy = dalloc<float>(static_cast<size_t>(count) * w[L]);
-    int32_t* dperm = dalloc<int32_t>(static_cast<size_t>(count));
-    double* dl = dalloc<double>(1 + std::max(o.epochs, 1));
-    auto release = [&] {
-      cudaFree(dx);
-      cudaFree(dy);
-      cudaFree(dperm);
-      cudaFree(dl);
-      d_loss = nullptr;
-    };
-    try {
-      B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * count * w[0], cudaMemcpyHostToDevice, stream));
-      B2P_CUDA(cudaMemcpyAsync(dy, y, sizeof(float) * count * w[L], cudaMemcpyHostToDevice, stream));
-      B2P_CUDA(cudaMemsetAsync(dl, 0, sizeof(double) * (1 + std::max(o.epochs, 1)), stream));
-      d_loss = dl;
-      std::mt19937_64 rng(o.seed);
-      std::vector<int32_t> perm(count);
-      int64_t t = 0;
-      for (int ep = 0; ep < o.epochs; ++ep) {
-        std::iota(perm.begin(), perm.end(), 0);
-        std::shuffle(perm.begin(), perm.end(), rng);
-        B2P_CUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, stream));
-        for (int64_t sidx = 0; sidx < steps_per_epoch; ++sidx, ++t) {
-          launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(bs) * (w[0] + w[L])), kEw, 0, stream, bs, w[0], w[L], dx,
-                     dy, dperm, sidx * bs, act[0], target);
-          forward(bs, out, stream);
-          loss_backward(bs, dl + 1 + ep, 1.0 / static_cast<double>(steps_per_epoch));
-          ++step;
-          const double frac = total > 1 ? static_cast<double>(t) / static_cast<double>(total - 1) : 1.0;
-          const double lr = o.lr_final + 0.5 * (o.lr - o.lr_final) * (1.0 + std::cos(M_PI * frac));
-          const double c1 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta1), static_cast<double>(step)));
-          const double c2 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta2), static_cast<double>(step)));
-          launch_pdl(k_adam, ew_blocks(nparams / 4), kEw, 0, stream, nparams / 4, reinterpret_cast<float4*>(params),
-                     reinterpret_cast<const float4*>(grads), reinterpret_cast<float4*>(adam_m),
-                     reinterpret_cast<float4*>(adam_v), reinterpret_cast<const uchar4*>(decay),
-                     static_cast<float>(lr), o.beta1, o.beta2, static_cast<float>(c1), static_cast<float>(c2), o.eps,
-                     o.weight_decay, reinterpret_cast<uint2*>(pbf));
-        }
+    CallBuffers buf(device, stream);
+    float* dx = buf.get<float>(static_cast<size_t>(count) * w[0]);
+    float* dy = buf.get<float>(static_cast<size_t>(count) * w[L]);
+    int32_t* dperm = buf.get<int32_t>(static_cast<size_t>(count));
+    double* dl = buf.get<double>(1 + std::max(o.epochs, 1));
+    LossGuard guard{*this, dl};
+    B2P_CUDA(cudaMemcpyAsync(dx, x, sizeof(float) * count * w[0], cudaMemcpyHostToDevice, stream));
+    B2P_CUDA(cudaMemcpyAsync(dy, y, sizeof(float) * count * w[L], cudaMemcpyHostToDevice, stream));
+    B2P_CUDA(cudaMemsetAsync(dl, 0, sizeof(double) * (1 + std::max(o.epochs, 1)), stream));
+    std::mt19937_64 rng(o.seed);
+    std::vector<int32_t> perm(count);
+    int64_t t = 0;
+    for (int ep = 0; ep < o.epochs; ++ep) {
+      std::iota(perm.begin(), perm.end(), 0);
+      std::shuffle(perm.begin(), perm.end(), rng);
+      B2P_CUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, stream));
+      for (int64_t sidx = 0; sidx < steps_per_epoch; ++sidx, ++t) {
+        launch_pdl(k_gather, ew_blocks(static_cast<int64_t>(bs) * (w[0] + w[L])), kEw, 0, stream, bs, w[0], w[L], dx,
+                   dy, dperm, sidx * bs, act[0], target);
+        forward(bs, out, stream);
+        loss_backward(bs, dl + 1 + ep, 1.0 / static_cast<double>(steps_per_epoch));
+        ++step;
+        const double frac = total > 1 ? static_cast<double>(t) / static_cast<double>(total - 1) : 1.0;
+        const double lr = o.lr_final + 0.5 * (o.lr - o.lr_final) * (1.0 + std::cos(M_PI * frac));
+        const double c1 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta1), static_cast<double>(step)));
+        const double c2 = 1.0 / (1.0 - std::pow(static_cast<double>(o.beta2), static_cast<double>(step)));
+        launch_pdl(k_adam, ew_blocks(nparams / 4), kEw, 0, stream, nparams / 4, reinterpret_cast<float4*>(params),
+                   reinterpret_cast<const float4*>(grads), reinterpret_cast<float4*>(adam_m),
+                   reinterpret_cast<float4*>(adam_v), reinterpret_cast<const uchar4*>(decay),
+                   static_cast<float>(lr), o.beta1, o.beta2, static_cast<float>(c1), static_cast<float>(c2), o.eps,
+                   o.weight_decay, reinterpret_cast<uint2*>(pbf));
       }
-      std::vector<double> hl(1 + std::max(o.epochs, 1));
-      B2P_CUDA(cudaMemcpyAsync(hl.data(), dl, sizeof(double) * hl.size(), cudaMemcpyDeviceToHost, stream));
-      check_error();
-      if (epoch_loss)
-        for (int ep = 0; ep < o.epochs; ++ep) epoch_loss[ep] = static_cast<float>(hl[1 + ep]);
-    } catch (...) {
-      release();
-      throw;
     }
-    release();
+    std::vector<double> hl(1 + std::max(o.epochs, 1));
+    B2P_CUDA(cudaMemcpyAsync(hl.data(), dl, sizeof(double) * hl.size(), cudaMemcpyDeviceToHost, stream));
+    check_error();
+    if (epoch_loss)
+      for (int ep = 0; ep < o.epochs; ++ep) epoch_loss[ep] = static_cast<float>(hl[1 + ep]);
   }
 };
 
@@ -738,39 +752,34 @@ int b2p_mlp_gemm_bf16(int32_t M, int32_t N, int32_t K, const uint16_t* A, int64_
     if (major != 10) throw Error(B2P_ERR_NO_DEVICE, "tcgen05 GEMM needs an sm_100 device");
     set_gemm_attributes();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int32_t* derr = dalloc<int32_t>(1);
+    ErrorWord error;
+    GemmArgs g{};
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.A = reinterpret_cast<const __nv_bfloat16*>(A);
+    g.sam = sam;
+    g.sak = sak;
+    g.B = reinterpret_cast<const __nv_bfloat16*>(B);
+    g.sbk = sbk;
+    g.sbn = sbn;
+    g.alpha = alpha;
+    g.bias = bias;
+    g.relu = relu;
+    g.mask = reinterpret_cast<const __nv_bfloat16*>(mask);
+    g.ldm = ldm;
+    g.cf = cf;
+    g.ldcf = ldcf;
+    g.cb = reinterpret_cast<__nv_bfloat16*>(cb);
+    g.ldcb = ldcb;
+    g.error = error.device();
     try {
-      B2P_CUDA(cudaMemsetAsync(derr, 0, sizeof(int32_t), s));
-      GemmArgs g{};
-      g.M = M;
-      g.N = N;
-      g.K = K;
-      g.A = reinterpret_cast<const __nv_bfloat16*>(A);
-      g.sam = sam;
-      g.sak = sak;
-      g.B = reinterpret_cast<const __nv_bfloat16*>(B);
-      g.sbk = sbk;
-      g.sbn = sbn;
-      g.alpha = alpha;
-      g.bias = bias;
-      g.relu = relu;
-      g.mask = reinterpret_cast<const __nv_bfloat16*>(mask);
-      g.ldm = ldm;
-      g.cf = cf;
-      g.ldcf = ldcf;
-      g.cb = reinterpret_cast<__nv_bfloat16*>(cb);
-      g.ldcb = ldcb;
-      g.error = derr;
       launch_gemm(g, s);
-      int32_t h = 0;
-      B2P_CUDA(cudaMemcpyAsync(&h, derr, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      B2P_CUDA(cudaStreamSynchronize(s));
-      if (h) throw Error(B2P_ERR_CUDA, "tensor-core GEMM: mbarrier wait timed out");
+      error.check(s);
     } catch (...) {
-      cudaFree(derr);
+      cudaStreamSynchronize(s);  // nothing still writes the word when it goes back
       throw;
     }
-    cudaFree(derr);
   });
 }
 
@@ -787,24 +796,20 @@ int b2p_mlp_gemm_bf16_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, i
     set_gemm_attributes();
     cudaStream_t s = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    int32_t* derr = nullptr;
+    ErrorWord error;
     struct Cleanup {
       cudaStream_t& s;
       cudaEvent_t &e0, &e1;
-      int32_t*& derr;
       ~Cleanup() {
         if (s) cudaStreamSynchronize(s);
-        if (derr) cudaFree(derr);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (s) cudaStreamDestroy(s);
       }
-    } cleanup{s, e0, e1, derr};
+    } cleanup{s, e0, e1};
     B2P_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     B2P_CUDA(cudaEventCreate(&e0));
     B2P_CUDA(cudaEventCreate(&e1));
-    derr = dalloc<int32_t>(1);
-    B2P_CUDA(cudaMemsetAsync(derr, 0, sizeof(int32_t), s));
     GemmArgs g{};
     g.M = M;
     g.N = N;
@@ -818,7 +823,7 @@ int b2p_mlp_gemm_bf16_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, i
     g.alpha = 1.0f;
     g.cf = cf;
     g.ldcf = ldcf;
-    g.error = derr;
+    g.error = error.device();
     launch_gemm(g, s);  // warm-up (module load, attributes)
     B2P_CUDA(cudaEventRecord(e0, s));
     for (int r = 0; r < reps; ++r) launch_gemm(g, s);
@@ -826,10 +831,7 @@ int b2p_mlp_gemm_bf16_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, i
     B2P_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
     B2P_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    int32_t h = 0;
-    B2P_CUDA(cudaMemcpyAsync(&h, derr, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    B2P_CUDA(cudaStreamSynchronize(s));
-    if (h) throw Error(B2P_ERR_CUDA, "tensor-core GEMM: mbarrier wait timed out");
+    error.check(s);
     *ms_per_launch = static_cast<double>(ms) / reps;
   });
 }

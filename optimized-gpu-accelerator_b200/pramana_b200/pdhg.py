@@ -148,22 +148,41 @@ class PdhgResult:
     primalWeight: float = 0.0
 
 
+# The C structs of many LPs and their results as one array each: filling a
+# ctypes structure field by field costs about 20 us an LP.
+_LP_DTYPE = np.dtype({"names": [f for f, _ in _lib.B2pLp._fields_],
+                      "formats": [{C.c_int32: "i4", C.c_double: "f8"}.get(t, "u8") for _, t in _lib.B2pLp._fields_],
+                      "offsets": [getattr(_lib.B2pLp, f).offset for f, _ in _lib.B2pLp._fields_],
+                      "itemsize": C.sizeof(_lib.B2pLp)})
+_RESULT_DTYPE = np.dtype({"names": [f for f, _ in _lib.B2pResult._fields_],
+                          "formats": [{C.c_int32: "i4", C.c_int64: "i8"}.get(t, "f8")
+                                      for _, t in _lib.B2pResult._fields_],
+                          "offsets": [getattr(_lib.B2pResult, f).offset for f, _ in _lib.B2pResult._fields_],
+                          "itemsize": C.sizeof(_lib.B2pResult)})
+
+
+def _address(a) -> int:
+    return a.__array_interface__["data"][0]
+
+
+def _lp_record(lp: Model, keep: list) -> tuple:
+    """One LP as a record of _LP_DTYPE.  The arrays the addresses point into
+    are Model's own (a copy, kept alive in `keep`, where a field was replaced
+    by one of another type after construction)."""
+    at = []
+    for name, dtype in (("start", np.int32), ("index", np.int32), ("value", np.float64), ("col_cost", np.float64),
+                        ("col_lower", np.float64), ("col_upper", np.float64), ("row_lower", np.float64),
+                        ("row_upper", np.float64)):
+        a = np.ascontiguousarray(getattr(lp, name), dtype=dtype)
+        keep.append(a)
+        at.append(_address(a))
+    return (lp.num_rows, lp.num_cols, *at, float(lp.obj_offset))
+
+
 def _lp_struct(lp: Model):
     keep = []
-
-    def p(a, ctype):
-        # a no-op for the arrays Model already holds; a copy if a field was
-        # replaced by one of another dtype after construction
-        a = np.ascontiguousarray(a, dtype=np.int32 if ctype is C.c_int32 else np.float64)
-        keep.append(a)
-        return a.ctypes.data_as(C.POINTER(ctype))
-
-    s = _lib.B2pLp(num_rows=lp.num_rows, num_cols=lp.num_cols, start=p(lp.start, C.c_int32),
-                   index=p(lp.index, C.c_int32), value=p(lp.value, C.c_double), col_cost=p(lp.col_cost, C.c_double),
-                   col_lower=p(lp.col_lower, C.c_double), col_upper=p(lp.col_upper, C.c_double),
-                   row_lower=p(lp.row_lower, C.c_double), row_upper=p(lp.row_upper, C.c_double),
-                   obj_offset=float(lp.obj_offset))
-    return s, keep
+    record = np.array([_lp_record(lp, keep)], dtype=_LP_DTYPE)
+    return _lib.B2pLp.from_buffer_copy(record.tobytes()), keep
 
 
 def _cases_struct(cases, n, m):
@@ -199,12 +218,15 @@ def _device_name() -> str:
     return _DEVICE_NAME[0]
 
 
-def _results(lp: Model, res, x, y, k, stats) -> list[PdhgResult]:
-    n, m = lp.num_cols, lp.num_rows
-    return [PdhgResult(status=Status.get(res[b].status, str(res[b].status)), objective=res[b].objective,
-                       dualObjective=res[b].dual_objective, x=x[b * n:(b + 1) * n].copy(),
-                       rowDual=y[b * m:(b + 1) * m].copy(), iterations=res[b].iterations,
-                       relativeKkt=res[b].relative_kkt, stats=stats) for b in range(k)]
+def _results(res, xs, ys, stats, weights=None) -> list[PdhgResult]:
+    """Result b of the records `res` with its arrays xs[b] and ys[b]."""
+    r = np.frombuffer(res, dtype=_RESULT_DTYPE)
+    weights = [0.0] * len(r) if weights is None else weights.tolist()
+    return [PdhgResult(status=Status.get(st, str(st)), objective=po, dualObjective=do, x=x, rowDual=y, iterations=it,
+                       relativeKkt=kkt, stats=stats, primalWeight=w)
+            for st, po, do, x, y, it, kkt, w in zip(r["status"].tolist(), r["objective"].tolist(),
+                                                    r["dual_objective"].tolist(), xs, ys, r["iterations"].tolist(),
+                                                    r["relative_kkt"].tolist(), weights)]
 
 
 def solvePdhg(lp: Model, opts: PdhgOptions | None = None, cancel_flag=None) -> PdhgResult:
@@ -220,7 +242,7 @@ def solvePdhg(lp: Model, opts: PdhgOptions | None = None, cancel_flag=None) -> P
     _lib.check(lib.b2p_solve_pdhg(C.byref(s), C.byref(o), x.ctypes.data_as(_lib.dptr), y.ctypes.data_as(_lib.dptr),
                                   res, C.byref(st)))
     del keep
-    return _results(lp, res, x, y, 1, PdhgStats.from_c(st, _device_name()))[0]
+    return _results(res, [x], [y], PdhgStats.from_c(st, _device_name()))[0]
 
 
 def solvePdhgBatch(base: Model, cases: list[LpCase], opts: PdhgOptions | None = None,
@@ -244,7 +266,7 @@ def solvePdhgBatch(base: Model, cases: list[LpCase], opts: PdhgOptions | None = 
     stats = PdhgStats.from_c(st, _device_name())
     if batchStats is not None:
         batchStats.__dict__.update(stats.__dict__)
-    return _results(base, res, x, y, k, stats)
+    return _results(res, x.reshape(k, base.num_cols), y.reshape(k, base.num_rows), stats)
 
 
 def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats: PdhgStats | None = None,
@@ -261,16 +283,16 @@ def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats
     opts = opts or PdhgOptions()
     lib = _lib.load()
     k = len(lps)
-    structs, keep = [], []
-    arr = (_lib.B2pLp * k)()
-    for b, lp in enumerate(lps):
-        s, kp = _lp_struct(lp)
-        arr[b] = s
-        keep.append(kp)
-    xs = [np.zeros(lp.num_cols) for lp in lps]
-    ys = [np.zeros(lp.num_rows) for lp in lps]
-    xp = (_lib.dptr * k)(*[a.ctypes.data_as(_lib.dptr) for a in xs])
-    yp = (_lib.dptr * k)(*[a.ctypes.data_as(_lib.dptr) for a in ys])
+    keep: list = []
+    arr = np.array([_lp_record(lp, keep) for lp in lps], dtype=_LP_DTYPE)
+    # every LP's answer in one buffer, its result a view of it
+    col = np.cumsum([0] + [lp.num_cols for lp in lps])
+    row = np.cumsum([0] + [lp.num_rows for lp in lps])
+    xall, yall = np.zeros(col[-1]), np.zeros(row[-1])
+    xs = [xall[i:j] for i, j in zip(col[:-1].tolist(), col[1:].tolist())]
+    ys = [yall[i:j] for i, j in zip(row[:-1].tolist(), row[1:].tolist())]
+    xp = (_address(xall) + 8 * col[:-1]).astype(np.uint64)
+    yp = (_address(yall) + 8 * row[:-1]).astype(np.uint64)
     res = (_lib.B2pResult * k)()
     st = _lib.B2pStats()
     o = opts.to_c(cancel_flag)
@@ -286,18 +308,17 @@ def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats
         w_in = np.ascontiguousarray(np.asarray(primalWeights, dtype=np.float64).reshape(k))
         keep.append(w_in)
     w_out = np.zeros(k)
-    _lib.check(lib.b2p_solve_pdhg_multi_warm(arr, k, C.byref(o), xst, yst,
-                                              None if w_in is None else w_in.ctypes.data_as(_lib.dptr), xp, yp,
+    pp = C.POINTER(_lib.dptr)
+    _lib.check(lib.b2p_solve_pdhg_multi_warm(arr.ctypes.data_as(C.POINTER(_lib.B2pLp)), k, C.byref(o), xst, yst,
+                                              None if w_in is None else w_in.ctypes.data_as(_lib.dptr),
+                                              xp.ctypes.data_as(pp), yp.ctypes.data_as(pp),
                                               w_out.ctypes.data_as(_lib.dptr), res, C.byref(st)))
-    del keep, structs
+    del keep
     stats = PdhgStats.from_c(st, _device_name())
     if batchStats is not None:
         batchStats.__dict__.update(stats.__dict__)
     solvePdhgMulti.last_stats = st
-    return [PdhgResult(status=Status.get(res[b].status, str(res[b].status)), objective=res[b].objective,
-                       dualObjective=res[b].dual_objective, x=xs[b], rowDual=ys[b], iterations=res[b].iterations,
-                       relativeKkt=res[b].relative_kkt, stats=stats, primalWeight=float(w_out[b]))
-            for b in range(k)]
+    return _results(res, xs, ys, stats, w_out)
 
 
 def gpuAvailable() -> bool:
@@ -341,7 +362,8 @@ class Engine:
         _lib.check(self._lib.b2p_engine_solve(self._h, res, C.byref(st)))
         self.last_stats = st
         x, y = self.fetch()
-        return _results(self.lp, res, x, y, self.k, PdhgStats.from_c(st))
+        return _results(res, x.reshape(self.k, self.lp.num_cols), y.reshape(self.k, self.lp.num_rows),
+                        PdhgStats.from_c(st))
 
     def set_start(self, x=None, y=None, primal_weight: float = 0.0) -> None:
         """Warm start of the following solves (original space); None, None = cold start."""
