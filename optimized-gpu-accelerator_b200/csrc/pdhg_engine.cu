@@ -118,6 +118,39 @@ __global__ void __launch_bounds__(kBlock) k_pack_cases(int64_t rows, int32_t k, 
   dst[t] = src[r * k + map[t - r * k2]];
 }
 
+// Answers of some cases: dst[to[q] * rows + r] = src[r * k + from[q]] *
+// fac[r] * scale, q < count -- out of the k-interleaved scaled space into the
+// caller's order and units (src/pdhg/pdhg.cpp:571-587).  32 x 32 tiles through
+// shared memory, so that both sides move whole sectors.  Beside the D2H copies
+// this is all an answer costs; unscaled and de-interleaved on the host after
+// every check at which a case ended, the 256-case sweep of the large refinery
+// (33 MB of answers) spent 35 of 87 ms a solve there.
+constexpr int kAnswerTile = 32;
+__global__ void __launch_bounds__(kBlock) k_answers(int32_t rows, int32_t k, int32_t count,
+                                                    const int32_t* __restrict__ from, const int32_t* __restrict__ to,
+                                                    const double* __restrict__ src, const double* __restrict__ fac,
+                                                    double scale, double* __restrict__ dst) {
+  __shared__ double tile[kAnswerTile][kAnswerTile + 1];
+  constexpr int kStep = kBlock / kAnswerTile;
+  const int lane = threadIdx.x % kAnswerTile, sub = threadIdx.x / kAnswerTile;
+  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kAnswerTile;
+  const int q0 = blockIdx.y * kAnswerTile;
+  if (q0 + lane < count) {
+    const int b = from[q0 + lane];
+#pragma unroll
+    for (int i = sub; i < kAnswerTile; i += kStep)
+      if (r0 + i < rows) tile[i][lane] = src[(r0 + i) * k + b];
+  }
+  __syncthreads();
+  const int64_t r = r0 + lane;
+  if (r >= rows) return;
+  const double f = fac[r];
+#pragma unroll
+  for (int i = sub; i < kAnswerTile; i += kStep)
+    if (q0 + i < count)
+      dst[static_cast<int64_t>(to[q0 + i]) * rows + r] = __dmul_rn(__dmul_rn(tile[lane][i], f), scale);
+}
+
 struct Engine {
   // ---- problem ----
   int device = 0;
@@ -135,6 +168,10 @@ struct Engine {
   std::vector<void*> allocs;
   int32_t *dA_ptr = nullptr, *dA_idx = nullptr, *dT_ptr = nullptr, *dT_idx = nullptr;
   double *dA_val = nullptr, *dT_val = nullptr, *d_rfac = nullptr, *d_cfac = nullptr;
+  double *d_rscale = nullptr, *d_cscale = nullptr;  // the scaling factors R and Cs
+  double *d_xans = nullptr, *d_yans = nullptr;      // answers: num_cases x n / x m, original space
+  int32_t* d_ended = nullptr;                       // cases whose answers are taken: packed index, then the engine's
+  bool solved = false;                              // the answers are a solve's
   double* v[NSLOT] = {};
   // Case compaction of a batch (FP64 phase): when half the live cases have
   // terminated, the rest are packed into a narrower interleave, so that the
@@ -190,7 +227,6 @@ struct Engine {
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
 
   // ---- last solve ----
-  std::vector<double> x_out, y_out;  // num_cases x n / x m, original space
   std::vector<b2p_result> results;
   b2p_stats stats{};
   int64_t launches = 0;
@@ -326,6 +362,11 @@ struct Engine {
     eta = 0.998 / P.normA;
     d_rfac = upload(P.rfac);
     d_cfac = upload(P.cfac);
+    d_rscale = upload(P.R);
+    d_cscale = upload(P.Cs);
+    d_xans = dalloc<double>(nk);
+    d_yans = dalloc<double>(mk);
+    d_ended = dalloc<int32_t>(static_cast<size_t>(2) * k);
     if (k == 1) {
       const auto tk = Clock::now();
       int per_sm = 0;
@@ -1074,17 +1115,36 @@ struct Engine {
     }
   }
 
-  void download_iterates(std::vector<double>& xs, std::vector<double>& ys) {
+  // x+ and y+ of the packed cases `ended` into the answers.
+  void take_answers(const std::vector<int32_t>& ended) {
+    if (ended.empty()) return;
+    const int count = static_cast<int>(ended.size());
+    std::vector<int32_t> list(ended);
+    for (int32_t b : ended) list.push_back(case_of[b]);
+    B2P_CUDA(cudaMemcpyAsync(d_ended, list.data(), sizeof(int32_t) * list.size(), cudaMemcpyHostToDevice, stream));
+    const auto part = [&](int64_t rows, const double* src, const double* fac, double scale, double* dst) {
+      if (rows)
+        k_answers<<<dim3(static_cast<unsigned>((rows + kAnswerTile - 1) / kAnswerTile),
+                         static_cast<unsigned>((count + kAnswerTile - 1) / kAnswerTile)),
+                    kBlock, 0, stream>>>(static_cast<int32_t>(rows), k, count, d_ended, d_ended + count, src, fac, scale,
+                                         dst);
+    };
+    part(n, v[XP], d_cscale, P.beta, d_xans);
+    part(m, v[YP], d_rscale, P.gamma, d_yans);
+    B2P_CUDA(cudaGetLastError());
+  }
+
+  // The last solve's answers (none before the first).
+  void fetch(double* x, double* y) {
+    if (!solved) return;
     const auto t0 = Clock::now();
-    xs.resize(static_cast<size_t>(n) * k);
-    ys.resize(static_cast<size_t>(m) * k);
-    if (!xs.empty())
-      B2P_CUDA(cudaMemcpyAsync(xs.data(), v[XP], xs.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    if (!ys.empty())
-      B2P_CUDA(cudaMemcpyAsync(ys.data(), v[YP], ys.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    B2P_CUDA(cudaSetDevice(device));
+    const size_t nk = static_cast<size_t>(n) * k, mk = static_cast<size_t>(m) * k;
+    if (x && nk) B2P_CUDA(cudaMemcpyAsync(x, d_xans, nk * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    if (y && mk) B2P_CUDA(cudaMemcpyAsync(y, d_yans, mk * sizeof(double), cudaMemcpyDeviceToHost, stream));
     B2P_CUDA(cudaStreamSynchronize(stream));
-    bytes_down += static_cast<int64_t>((xs.size() + ys.size()) * sizeof(double));
     transfer_seconds += seconds_since(t0);
+    stats.transfer_seconds = transfer_seconds;
   }
 
   void drop_graphs() {
@@ -1175,12 +1235,11 @@ struct Engine {
     int stale32 = 0;
     constexpr int kStallChecks = 20;
     results.assign(k, b2p_result{});
-    x_out.assign(static_cast<size_t>(n) * k, 0.0);
-    y_out.assign(static_cast<size_t>(m) * k, 0.0);
+    solved = false;
     stats.restarts = 0;
     std::vector<char> done(k, 0);
     std::vector<RestartTracker> restarts(k);
-    std::vector<double> xs, ys;
+    std::vector<int32_t> ended;  // packed cases that end at this check
     int remaining = k;
     int checks = 0;
     const double scaleObj = P.beta * P.gamma;
@@ -1190,10 +1249,8 @@ struct Engine {
       return opt.time_limit > 0 && seconds_since(deadline_start) >= opt.time_limit;
     };
     auto extract = [&](int b, int status, double relKkt, double pobj, double dobj, int64_t it) {
-      const size_t cb = static_cast<size_t>(case_of[b]);
-      for (int j = 0; j < n; ++j) x_out[cb * n + j] = xs[static_cast<size_t>(j) * k + b] * P.Cs[j] * P.beta;
-      for (int i = 0; i < m; ++i) y_out[cb * m + i] = ys[static_cast<size_t>(i) * k + b] * P.R[i] * P.gamma;
-      b2p_result& r = results[cb];
+      ended.push_back(b);
+      b2p_result& r = results[case_of[b]];
       r.status = status;
       r.iterations = it;
       r.relative_kkt = relKkt;
@@ -1214,7 +1271,8 @@ struct Engine {
       if (phase32) stats.fp32_iterations += L;
       it += L - 1;  // index of the check iteration
       ++checks;
-      bool anyRestart = false, fetched = false;
+      bool anyRestart = false;
+      ended.clear();
       for (int b = 0; b < k; ++b) h_mask[b] = 0;
       if (phase32 && mixed_batch) {
         // Mixed form of a batch: each case's FP32 point is measured in FP64
@@ -1245,7 +1303,6 @@ struct Engine {
         if (ready) {
           fp32_point_to_fp64();
           verify_fp64();
-          bool fetched64 = false;
           for (int b = 0; b < k; ++b) {
             if (done[b]) continue;
             const double* s = h_sums + static_cast<size_t>(b) * kNumSums;
@@ -1254,15 +1311,12 @@ struct Engine {
             const double relD = std::sqrt(s[CS_COL_RES2]) / (1.0 + cn[b]);
             const double gap = std::fabs(pobj - dobj) / (1.0 + std::fabs(pobj) + std::fabs(dobj));
             if (relP <= opt.tolerance && relD <= opt.tolerance && gap <= opt.tolerance) {
-              if (!fetched64) {
-                download_iterates(xs, ys);
-                fetched64 = true;
-              }
               extract(b, B2P_STATUS_OPTIMAL, smax(relP, smax(relD, gap)), pobj, dobj, it);
               done[b] = 1;
               --remaining;
             }
           }
+          take_answers(ended);
           if (remaining == 0) break;
           switch_to_fp64();
           for (auto& r : restarts) r.reset();
@@ -1298,8 +1352,8 @@ struct Engine {
           stats.dual_residual = vrelD;
           stats.gap = vgap;
           if (vrelP <= opt.tolerance && vrelD <= opt.tolerance && vgap <= opt.tolerance) {
-            download_iterates(xs, ys);
             extract(0, B2P_STATUS_OPTIMAL, smax(vrelP, smax(vrelD, vgap)), vpobj, vdobj, it);
+            take_answers(ended);
             done[0] = 1;
             remaining = 0;
             break;
@@ -1343,10 +1397,6 @@ struct Engine {
                        static_cast<long long>(it + 1), pobj + P.offset, dobj + P.offset, relP, relD, gap, omega[b],
                        stats.restarts, seconds_since(t_solve));
         if (!phase32 && relP <= opt.tolerance && relD <= opt.tolerance && gap <= opt.tolerance) {
-          if (!fetched) {
-            download_iterates(xs, ys);
-            fetched = true;
-          }
           extract(b, B2P_STATUS_OPTIMAL, kktErr, pobj, dobj, it);
           done[b] = 1;
           --remaining;
@@ -1357,6 +1407,7 @@ struct Engine {
           anyRestart = true;
         }
       }
+      take_answers(ended);
       if (anyRestart) {
         for (int b = 0; b < k; ++b) {
           if (!h_mask[b]) continue;
@@ -1427,7 +1478,7 @@ struct Engine {
         fp32_point_to_fp64();
         verify_fp64();
       }
-      download_iterates(xs, ys);
+      ended.clear();
       for (int b = 0; b < k; ++b) {
         if (done[b]) continue;
         const double* s = h_sums + static_cast<size_t>(b) * kNumSums;
@@ -1438,7 +1489,10 @@ struct Engine {
         extract(b, (expiredStop || expired()) ? B2P_STATUS_TIME_LIMIT : B2P_STATUS_ITERATION_LIMIT,
                 smax(relP, smax(relD, gap)), pobj, dobj, it);
       }
+      take_answers(ended);
     }
+    solved = true;
+    bytes_down += static_cast<int64_t>(sizeof(double)) * (static_cast<int64_t>(n) + m) * k_full;  // fetch
     stats.kernel_launches = launches;
     stats.bytes_uploaded = bytes_up;
     stats.bytes_downloaded = bytes_down;
@@ -1472,8 +1526,7 @@ using b2p::guarded;
 namespace {
 
 void copy_results(Engine& e, double* x, double* y, b2p_result* results, b2p_stats* stats) {
-  if (x && !e.x_out.empty()) std::memcpy(x, e.x_out.data(), e.x_out.size() * sizeof(double));
-  if (y && !e.y_out.empty()) std::memcpy(y, e.y_out.data(), e.y_out.size() * sizeof(double));
+  if (x || y) e.fetch(x, y);
   if (results) std::memcpy(results, e.results.data(), e.results.size() * sizeof(b2p_result));
   if (stats) *stats = e.stats;
 }
