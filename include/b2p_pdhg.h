@@ -159,7 +159,7 @@ typedef struct b2p_options {
   int32_t cta_kernel;
   /* FP64 batches (k > 1 cases sharing A): variant of the two per-iteration
    * kernels -- 0 = timed on the device when the batch's vectors far exceed L2
-   * (plain otherwise); 1..4 force (cases per thread, evict-first streamed
+   * (chosen by size otherwise); 1..4 force (cases per thread, evict-first streamed
    * vectors) = (1, no), (2, no), (1, yes), (2, yes); 5..8 the same with whole
    * warps per row (row entries loaded once per warp and shared by shuffle)
    * where k / cases per thread is a multiple of 32; 9..16, 17..24 and 25..32

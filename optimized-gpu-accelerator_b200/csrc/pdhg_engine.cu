@@ -215,11 +215,17 @@ struct Engine {
   std::map<int, cudaGraphExec_t> graphs, graphs32;  // per interval length; FP32 phase of a batch
   std::map<int, cudaGraph_t> graph_defs, graph_defs32;
   bool mixed_batch = false;  // mixed form of a batch (k > 1): FP32 k-interleaved kernels
-  bool batch_stream_p = false, batch_stream_d = false;  // evict-first streamed vectors (tuned per kernel)
-  int batch_cpt_p = 1, batch_cpt_d = 1;  // cases per thread of the primal / dual batch kernels (tuned)
-  bool batch_wr_p = false, batch_wr_d = false;  // whole warps per row, entries passed by shuffle (tuned)
-  bool batch_wr_p_full = false, batch_wr_d_full = false;  // the tuned choice, restored after a compaction
-  int batch_tr_p = 0, batch_tr_d = 0;  // rows per block of the row-tiled layout (0 = one row's cases per block; tuned)
+  // Variant of an FP64 batch kernel: evict-first streamed vectors, cases per
+  // thread, whole warps per row (entries passed by shuffle), rows per block of
+  // the row-tiled layout (0 = one row's cases per block).
+  struct BatchVariant {
+    bool stream = false;
+    int cpt = 1;
+    bool wr = false;
+    int tr = 0;
+  };
+  BatchVariant batch_p, batch_d;            // primal / dual kernel at the current width
+  BatchVariant batch_p_full, batch_d_full;  // at the engine's own width, restored after a compaction
   bool profiling = false;
   std::vector<cudaEvent_t> prof_ev;  // 4 per iteration of the longest interval
   int64_t prof_launches[5] = {0, 0, 0, 0, 0};
@@ -884,7 +890,7 @@ struct Engine {
   // Row tiles of the batch kernels' layouts (0 = one row's cases per block).
   static constexpr int kTileRows[4] = {0, 4, 8, 16};
 
-  // FP64 batch kernel variants: forced by the options, or, for batches whose
+  // FP64 batch kernel variants: forced by the options, by size (batch_rule), or, for batches whose
   // vectors far exceed L2 (k (m + n) >= 2^22 elements), each kernel is timed
   // with one and with two cases per thread, with and (when k / cases per
   // thread is a multiple of 32) without per-lane index loads, with cached and
@@ -897,23 +903,41 @@ struct Engine {
     if (opt.batch_variant > 0) {
       const int w = (opt.batch_variant - 1) % 8 + 1;  // the layout-free part, 1..8
       const int v0 = (w - 1) % 4 + 1;
-      batch_cpt_p = batch_cpt_d = (v0 == 2 || v0 == 4) ? 2 : 1;
-      batch_stream_p = batch_stream_d = v0 >= 3;
-      batch_wr_p = batch_wr_d = w > 4 && warp_rows(batch_cpt_p);
-      batch_tr_p = batch_tr_d = kTileRows[(opt.batch_variant - 1) / 8];
+      batch_p.cpt = (v0 == 2 || v0 == 4) ? 2 : 1;
+      batch_p.stream = v0 >= 3;
+      batch_p.wr = w > 4 && warp_rows(batch_p.cpt);
+      batch_p.tr = kTileRows[(opt.batch_variant - 1) / 8];
+      batch_d = batch_p;
     } else if (static_cast<int64_t>(n + m) * k >= (int64_t(1) << 22)) {
       time_batch_variants();
+    } else {
+      batch_p = batch_d = batch_rule();
     }
-    stats.streaming_at = batch_stream_p;
-    stats.streaming_a = batch_stream_d;
-    stats.cases_per_thread_at = batch_cpt_p;
-    stats.cases_per_thread_a = batch_cpt_d;
-    stats.warp_rows_at = batch_wr_p;
-    stats.warp_rows_a = batch_wr_d;
-    stats.tile_rows_at = batch_tr_p;
-    stats.tile_rows_a = batch_tr_d;
+    stats.streaming_at = batch_p.stream;
+    stats.streaming_a = batch_d.stream;
+    stats.cases_per_thread_at = batch_p.cpt;
+    stats.cases_per_thread_a = batch_d.cpt;
+    stats.warp_rows_at = batch_p.wr;
+    stats.warp_rows_a = batch_d.wr;
+    stats.tile_rows_at = batch_p.tr;
+    stats.tile_rows_a = batch_d.tr;
   }
 
+  // Variant by size alone, for batches not worth timing (and for what a
+  // compaction leaves).  Plain while the iteration's 17 vectors fit L2 (there
+  // the forms differ by less than runs of one form do).  Past that, streamed
+  // vectors (us per iteration of the large refinery, plain / streamed: 101
+  // cases, 1.66 M elements, 33.9 / 32.4; 128 43.5 / 39.1; 250 83.0 / 70.6),
+  // and row tiles of 4, whose rows share their gathers in L1, where the
+  // 32-case chunks leave at most 15 % of their lanes idle (streamed without /
+  // with tiles: 160 cases 47.1 / 42.8, 200 57.3 / 57.6; with 27 % idle, 101
+  // cases, 32.4 / 35.1).
+  BatchVariant batch_rule() const {
+    BatchVariant r;
+    r.stream = static_cast<int64_t>(n + m) * k >= 3 * (int64_t(1) << 19);
+    r.tr = r.stream && (k + 31) / 32 * 32 * 100 <= k * 115 ? 4 : 0;
+    return r;
+  }
   // Whole warps per row: k / cpt (rounded up) a multiple of 32.
   bool warp_rows(int cpt) const { return ((k + cpt - 1) / cpt) % 32 == 0; }
 
@@ -944,12 +968,12 @@ struct Engine {
             if (n) {
               const double t = timed([&] { enqueue_batch_primal(true, st != 0, ck, cpt, wr != 0, tr); });
               if (t < best_p)
-                best_p = t, batch_stream_p = st != 0, batch_cpt_p = cpt, batch_wr_p = wr != 0, batch_tr_p = tr;
+                best_p = t, batch_p = BatchVariant{st != 0, cpt, wr != 0, tr};
             }
             if (m) {
               const double t = timed([&] { enqueue_batch_dual(true, st != 0, ck, cpt, wr != 0, tr); });
               if (t < best_d)
-                best_d = t, batch_stream_d = st != 0, batch_cpt_d = cpt, batch_wr_d = wr != 0, batch_tr_d = tr;
+                best_d = t, batch_d = BatchVariant{st != 0, cpt, wr != 0, tr};
             }
           }
         }
@@ -969,10 +993,10 @@ struct Engine {
       const bool last = l == L - 1;
       const IterClock ck{d_it_base, d_restart_at, l};
       if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[4 * l + 0], stream));
-      if (nk) enqueue_batch_primal(!last, batch_stream_p, ck, batch_cpt_p, batch_wr_p, batch_tr_p);
+      if (nk) enqueue_batch_primal(!last, batch_p.stream, ck, batch_p.cpt, batch_p.wr, batch_p.tr);
       if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[4 * l + 1], stream));
       if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[4 * l + 2], stream));
-      if (mk) enqueue_batch_dual(!last, batch_stream_d, ck, batch_cpt_d, batch_wr_d, batch_tr_d);
+      if (mk) enqueue_batch_dual(!last, batch_d.stream, ck, batch_d.cpt, batch_d.wr, batch_d.tr);
       if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[4 * l + 3], stream));
       B2P_CUDA(cudaGetLastError());
     }
@@ -1183,9 +1207,10 @@ struct Engine {
     for (int q = 0; q < k2; ++q) co[q] = case_of[keep[q]];
     case_of = co;
     k = k2;
+    if (opt.batch_variant == 0) batch_p = batch_d = batch_rule();
     // whole-warp rows need k / (cases per thread) to be a multiple of 32
-    if (batch_wr_p && ((k + batch_cpt_p - 1) / batch_cpt_p) % 32 != 0) batch_wr_p = false;
-    if (batch_wr_d && ((k + batch_cpt_d - 1) / batch_cpt_d) % 32 != 0) batch_wr_d = false;
+    batch_p.wr = batch_p.wr && warp_rows(batch_p.cpt);
+    batch_d.wr = batch_d.wr && warp_rows(batch_d.cpt);
     drop_graphs();
     ++compactions;
     B2P_CUDA(cudaStreamSynchronize(stream));
@@ -1202,8 +1227,8 @@ struct Engine {
     k = k_full;
     case_of.resize(k);
     for (int b = 0; b < k; ++b) case_of[b] = b;
-    batch_wr_p = batch_wr_p_full;
-    batch_wr_d = batch_wr_d_full;
+    batch_p = batch_p_full;
+    batch_d = batch_d_full;
     drop_graphs();
     B2P_CUDA(cudaStreamSynchronize(stream));
   }
@@ -1212,8 +1237,8 @@ struct Engine {
   void solve(Clock::time_point deadline_start) {
     B2P_CUDA(cudaSetDevice(device));
     restore_cases();
-    batch_wr_p_full = batch_wr_p;
-    batch_wr_d_full = batch_wr_d;
+    batch_p_full = batch_p;
+    batch_d_full = batch_d;
     compactions = 0;
     std::vector<double> cn(cNorm), rn(rhsNorm);  // per packed case
     const auto t_solve = Clock::now();
