@@ -206,7 +206,7 @@ typedef struct b2p_stats {
   double prepare_seconds, upload_seconds, graph_seconds;
   int32_t lanes_per_row_a, lanes_per_row_at; /* schedule used */
   int32_t kernel_mode;                        /* B2P_KERNELS_FUSED or B2P_KERNELS_RESIDENT (batches: FUSED) */
-  int32_t resident_blocks;                    /* cooperative grid size in resident form */
+  int32_t resident_blocks;                    /* resident form: cooperative grid size, or blocks of the cluster a small LP runs on */
   int64_t resident_smem_bytes;                /* largest block's shared memory in resident form */
   int32_t precision_used;                     /* B2P_PRECISION_* actually run */
   int32_t batch_compactions;                  /* batches: times the live cases were packed narrower */

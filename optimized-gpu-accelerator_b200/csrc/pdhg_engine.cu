@@ -50,23 +50,23 @@ inline bool row_slot(int s) { return s >= Y; }
 template <class T>
 using ResidentFn = void (*)(ResidentArgs<T>);
 
-template <class T, int GC>
+template <class T, bool CLUSTER, int GC>
 ResidentFn<T> resident_fn_rows(int gr) {
   switch (gr) {
-    case 1: return k_resident<GC, 1, T>;
-    case 2: return k_resident<GC, 2, T>;
-    case 4: return k_resident<GC, 4, T>;
-    default: return k_resident<GC, 8, T>;
+    case 1: return k_resident<GC, 1, T, CLUSTER>;
+    case 2: return k_resident<GC, 2, T, CLUSTER>;
+    case 4: return k_resident<GC, 4, T, CLUSTER>;
+    default: return k_resident<GC, 8, T, CLUSTER>;
   }
 }
 
-template <class T>
+template <class T, bool CLUSTER>
 ResidentFn<T> resident_fn(int gc, int gr) {
   switch (gc) {
-    case 1: return resident_fn_rows<T, 1>(gr);
-    case 2: return resident_fn_rows<T, 2>(gr);
-    case 4: return resident_fn_rows<T, 4>(gr);
-    default: return resident_fn_rows<T, 8>(gr);
+    case 1: return resident_fn_rows<T, CLUSTER, 1>(gr);
+    case 2: return resident_fn_rows<T, CLUSTER, 2>(gr);
+    case 4: return resident_fn_rows<T, CLUSTER, 4>(gr);
+    default: return resident_fn_rows<T, CLUSTER, 8>(gr);
   }
 }
 
@@ -190,10 +190,13 @@ struct Engine {
   RowBins binsA{}, binsT{};  // k == 1 schedules of A and A^T
   // resident form
   bool resident = false;
+  bool cluster = false;  // on one cluster of kClusterBlocks blocks
+  static constexpr int kClusterBlocks = 8;
+  unsigned res_epoch = 0;  // grid barriers of the solve so far
   int res_blocks = 0, res_gc = 1, res_gr = 1;
   size_t res_smem = 0;
   int32_t *d_cb = nullptr, *d_rb = nullptr;
-  unsigned* d_sync = nullptr;  // arrive, generation, error flag
+  unsigned* d_sync = nullptr;  // arrivals, unused, error flag
   double* d_rpartial = nullptr;
   int32_t* h_error = nullptr;
   ResidentFn<double> res_fn = nullptr;
@@ -482,37 +485,48 @@ struct Engine {
     if (opt.kernel_mode == B2P_KERNELS_FUSED || n == 0 || m == 0) return;
     int optin = 0;
     B2P_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    const int nb = sms;
-    std::vector<int32_t> cb = balanced_split(P.AT, nb), rb = balanced_split(P.A, nb);
-    size_t need64 = 0, need32 = 0;
-    for (int b = 0; b < nb; ++b) {
-      const int nc = cb[b + 1] - cb[b], nr = rb[b + 1] - rb[b];
-      const int tn = P.AT.ptr[cb[b + 1]] - P.AT.ptr[cb[b]], an = P.A.ptr[rb[b + 1]] - P.A.ptr[rb[b]];
-      need64 = std::max(need64, resident_smem_bytes<double>(nc, nr, tn, an));
-      need32 = std::max(need32, resident_smem_bytes<float>(nc, nr, tn, an));
-    }
-    const size_t reserve = 1024;  // static shared memory of the kernel
+    std::vector<int32_t> cb = balanced_split(P.AT, sms), rb = balanced_split(P.A, sms);
+    // lanes per row, the same in both forms (so are the sums)
     res_gc = resident_lanes(P.AT, cb);
     res_gr = resident_lanes(P.A, rb);
+    const bool want32 = opt.precision == B2P_PRECISION_MIXED;
+    if (setup_cluster(optin, want32)) return;
+    size_t need64 = 0, need32 = 0;
+    slice_bytes(cb, rb, 0, need64, need32);
+    const size_t reserve = 1024;  // static shared memory of the kernel
     bool ok64 = need64 + reserve <= static_cast<size_t>(optin);
-    bool ok32 = opt.precision == B2P_PRECISION_MIXED && need32 + reserve <= static_cast<size_t>(optin);
-    if (ok64) {
-      res_fn = resident_fn<double>(res_gc, res_gr);
-      B2P_CUDA(cudaFuncSetAttribute(res_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(need64)));
+    bool ok32 = want32 && need32 + reserve <= static_cast<size_t>(optin);
+    const auto usable = [&](auto fn, size_t need) {
+      // the device's maximum, not this LP's need: the attribute is the
+      // function's, and another engine's launches may need more
+      B2P_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - static_cast<int>(reserve)));
       int per_sm = 0;
-      B2P_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, res_fn, kResidentThreads, need64));
-      ok64 = per_sm >= 1;
-    }
-    if (ok32) {
-      res_fn32 = resident_fn<float>(res_gc, res_gr);
-      B2P_CUDA(cudaFuncSetAttribute(res_fn32, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(need32)));
-      int per_sm = 0;
-      B2P_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, res_fn32, kResidentThreads, need32));
-      ok32 = per_sm >= 1;
-    }
+      B2P_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResidentThreads, need));
+      return per_sm >= 1;
+    };
+    if (ok64) ok64 = usable(res_fn = resident_fn<double, false>(res_gc, res_gr), need64);
+    if (ok32) ok32 = usable(res_fn32 = resident_fn<float, false>(res_gc, res_gr), need32);
     if (!ok64 && opt.kernel_mode == B2P_KERNELS_RESIDENT && !ok32)
       throw Error(B2P_ERR_TOO_LARGE, "LP does not fit the resident form (shared memory)");
     if (!ok64 && !ok32) return;
+    use_resident(cb, rb, ok64 ? need64 : 0, ok32 ? need32 : 0);
+  }
+
+  // Largest block's shared memory for a split, with `shared` exchanged entries
+  // held by every block.
+  void slice_bytes(const std::vector<int32_t>& cb, const std::vector<int32_t>& rb, int64_t shared, size_t& need64,
+                   size_t& need32) const {
+    need64 = need32 = 0;
+    for (size_t b = 0; b + 1 < cb.size(); ++b) {
+      const int nc = cb[b + 1] - cb[b], nr = rb[b + 1] - rb[b];
+      const int tn = P.AT.ptr[cb[b + 1]] - P.AT.ptr[cb[b]], an = P.A.ptr[rb[b + 1]] - P.A.ptr[rb[b]];
+      need64 = std::max(need64, resident_smem_bytes<double>(nc, nr, tn, an, shared));
+      need32 = std::max(need32, resident_smem_bytes<float>(nc, nr, tn, an, shared));
+    }
+  }
+
+  void use_resident(const std::vector<int32_t>& cb, const std::vector<int32_t>& rb, size_t smem64, size_t smem32) {
+    const int nb = static_cast<int>(cb.size()) - 1;
     d_cb = upload(cb);
     d_rb = upload(rb);
     d_sync = dalloc<unsigned>(4);
@@ -520,12 +534,59 @@ struct Engine {
     h_error = static_cast<int32_t*>(PinnedCache::get(sizeof(int32_t)));
     *h_error = 0;
     res_blocks = nb;
-    res_smem = ok64 ? need64 : 0;
-    res_smem32 = ok32 ? need32 : 0;
-    resident = ok64;
-    mixed = ok32;
+    res_smem = smem64;
+    res_smem32 = smem32;
+    resident = smem64 > 0;
+    mixed = smem32 > 0;
     stats.resident_blocks = nb;
-    stats.resident_smem_bytes = static_cast<int64_t>(ok64 ? need64 : need32);
+    stats.resident_smem_bytes = static_cast<int64_t>(resident ? smem64 : smem32);
+  }
+
+  // The cluster form, for every LP whose slices and exchanged vectors fit the
+  // shared memory of 8 blocks (the largest portable cluster; up to about
+  // 28,000 nonzeros).  It was faster than the grid form at every size that
+  // fits (us per iteration, clusters of 2 / 4 / 8 / 16 blocks against the
+  // grid's 148: 1,000 nonzeros 2.83 / 2.84 / 2.85 / 3.04 against 5.17, 10,000
+  // - / 4.12 / 3.62 / 3.86 against 5.74, 20,000 - / - / 4.82 / 4.96 against
+  // 5.78); 16 blocks would take up to 40,000 nonzeros, but there every block
+  // storing to 15 others costs more than the grid's barrier (6.43 / 5.72).
+  bool setup_cluster(int optin, bool want32) {
+    const std::vector<int32_t> cb = balanced_split(P.AT, kClusterBlocks), rb = balanced_split(P.A, kClusterBlocks);
+    size_t need64 = 0, need32 = 0;
+    slice_bytes(cb, rb, static_cast<int64_t>(n) + m, need64, need32);
+    const int most = optin - 1024;  // less the kernel's static shared memory
+    const auto usable = [&](auto fn, size_t need) {
+      if (need > static_cast<size_t>(most)) return false;
+      B2P_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      cluster_config(cfg, attr, need);
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      return clusters >= 1;
+    };
+    const bool ok64 = usable(res_fn = resident_fn<double, true>(res_gc, res_gr), need64);
+    const bool ok32 = want32 && usable(res_fn32 = resident_fn<float, true>(res_gc, res_gr), need32);
+    // both phases of a mixed solve run in one form
+    if (!ok64 || (want32 && !ok32)) return false;
+    cluster = true;
+    use_resident(cb, rb, need64, ok32 ? need32 : 0);
+    return true;
+  }
+
+  void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, size_t smem) const {
+    cfg.gridDim = dim3(kClusterBlocks);
+    cfg.blockDim = dim3(kResidentThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kClusterBlocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
   }
 
   // FP32 copies of the operators and case vectors for the mixed form.
@@ -550,7 +611,6 @@ struct Engine {
 
   template <class T>
   void launch_resident(int L, ResidentFn<T> fn, size_t smem, const T* a_val, const T* t_val, T* const* vs) {
-    B2P_CUDA(cudaMemsetAsync(d_sync, 0, 4 * sizeof(unsigned), stream));
     ResidentArgs<T> ra{};
     ra.cb = d_cb;
     ra.rb = d_rb;
@@ -594,15 +654,26 @@ struct Engine {
     ra.gen = d_sync + 1;
     ra.error = reinterpret_cast<int32_t*>(d_sync + 2);
     ra.partial = d_rpartial;
-    ra.sums = d_sums;
+    // the sums and the outcome go straight to the host's page-locked words
+    ra.sums = h_sums;
+    ra.failed = h_error;
     ra.it_base = d_it_base;
-    void* args[] = {&ra};
+    ra.epoch0 = res_epoch;
+    ra.m = m;
+    ra.n = n;
     if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[0], stream));
-    B2P_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(res_blocks), dim3(kResidentThreads), args,
-                                         smem, stream));
+    if (cluster) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      cluster_config(cfg, attr, smem);
+      B2P_CUDA(cudaLaunchKernelEx(&cfg, fn, ra));
+    } else {
+      void* args[] = {&ra};
+      B2P_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fn), dim3(res_blocks), dim3(kResidentThreads), args,
+                                           smem, stream));
+      res_epoch += 2 * static_cast<unsigned>(L) + 1;
+    }
     if (profiling) B2P_CUDA(cudaEventRecord(prof_ev[1], stream));
-    B2P_CUDA(cudaMemcpyAsync(h_sums, d_sums, sizeof(double) * kNumSums, cudaMemcpyDeviceToHost, stream));
-    B2P_CUDA(cudaMemcpyAsync(h_error, ra.error, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
   }
 
   void launch_resident64(int L) {
@@ -710,6 +781,8 @@ struct Engine {
     if (nk) B2P_CUDA(cudaMemsetAsync(v[XP], 0, nk * sizeof(double), stream));
     B2P_CUDA(cudaMemsetAsync(d_it_base, 0, sizeof(int64_t), stream));
     B2P_CUDA(cudaMemsetAsync(d_restart_at, 0, sizeof(int64_t) * k, stream));
+    if (d_sync) B2P_CUDA(cudaMemsetAsync(d_sync, 0, 4 * sizeof(unsigned), stream));
+    res_epoch = 0;
     omega = omega0;
     upload_steps(omega);
   }
