@@ -28,6 +28,7 @@
 
 #include "pdhg_host_common.h"
 #include "pdhg_kernels.cuh"
+#include "pdhg_members.cuh"
 #include "pdhg_ordered.cuh"
 #include "pdhg_prepare.h"
 #include "pdhg_restart.h"
@@ -312,6 +313,8 @@ enum MSlot : int { MX, MXP, MX0, MC, MLO, MUP, MXINIT, MATYP, MNCOL, MY = MNCOL,
 struct MultiEngine {
   int device = 0;
   int K = 0;
+  int ops = 0;         // operators held: K, or 1 for members of one operator in the CTA form
+  int32_t Mo = 0, No = 0;  // their rows and columns
   b2p_options opt{};
   std::vector<Prepared> P;
   std::vector<int64_t> roff, coff;  // row / column offsets of instance b
@@ -361,7 +364,9 @@ struct MultiEngine {
   b2p_stats stats{};
   std::vector<b2p_result> results;
   std::vector<double> weights;  // per LP: final primal weight, original-space units (omega gamma / beta)
-  std::vector<std::vector<double>> xs, ys;  // per instance, original space
+  MemberData md{};                                  // device: raw arrays, scaling factors
+  double* d_msums = nullptr;                        // kMemberSums per LP
+  double *d_xans = nullptr, *d_yans = nullptr;      // answers, original space
   int64_t launches = 0, bytes_up = 0, bytes_down = 0;
   int compactions = 0;
   // CTA form (pdhg_cta.cuh): one block per LP
@@ -409,8 +414,8 @@ struct MultiEngine {
     return d;
   }
   static unsigned blocks(int64_t len) { return static_cast<unsigned>(std::max<int64_t>(1, (len + kBlock - 1) / kBlock)); }
-  CsrView viewA() const { return CsrView{dA_ptr, dA_idx, dA_val, M}; }
-  CsrView viewAT() const { return CsrView{dT_ptr, dT_idx, dT_val, N}; }
+  CsrView viewA() const { return CsrView{dA_ptr, dA_idx, dA_val, Mo}; }
+  CsrView viewAT() const { return CsrView{dT_ptr, dT_idx, dT_val, No}; }
 
   ~MultiEngine() {
     for (auto& g : graphs) cudaGraphExecDestroy(g.second);
@@ -432,7 +437,12 @@ struct MultiEngine {
 
   void create(const b2p_lp* lps, int num, const b2p_options* o) {
     if (!lps || num <= 0) throw Error(B2P_ERR_INVALID, "no LPs");
-    for (int b = 0; b < num; ++b) check_lp(&lps[b]);
+    for (int b = 0; b < num; ++b) {
+      // an LP over the first one's column pointers and row indices: checked already
+      const bool same = b > 0 && lps[b].num_rows == lps[0].num_rows && lps[b].num_cols == lps[0].num_cols &&
+                        lps[b].start == lps[0].start && lps[b].index == lps[0].index && lps[b].value;
+      check_lp(&lps[b], !same);
+    }
     if (o) opt = *o; else b2p_default_options(&opt);
     if (opt.check_every <= 0) throw Error(B2P_ERR_INVALID, "check_every must be positive");
     device = pick_device(opt.device);
@@ -443,27 +453,41 @@ struct MultiEngine {
     K = num;
     shared_operator = same_operator(lps, num);
     const auto t0 = Clock::now();
-    // ---- host preparation of every instance (structure only), on all host threads ----
+    // Members of one operator in the CTA form, whose blocks read the first
+    // member's copy: only that one is prepared, uploaded and scaled.
+    const bool one = shared_operator && opt.multi_form != B2P_MULTI_GRID;
+    ops = one ? 1 : K;
+    // ---- host preparation of every operator (structure only), on all host threads ----
     P.resize(K);
-    std::atomic<int> next{0};
     const int nth = std::max(1u, std::min<unsigned>(std::thread::hardware_concurrency(), static_cast<unsigned>(K)));
-    std::vector<std::thread> pool;
-    std::vector<std::string> errs(nth);
-    for (int t = 0; t < nth; ++t)
-      pool.emplace_back([&, t] {
-        try {
-          for (int b; (b = next.fetch_add(1)) < K;) {
-            const b2p_lp& l = lps[b];
-            // structure and raw values; the scaling runs on the device below
-            P[b] = prepare_structure(l.num_rows, l.num_cols, l.start, l.index, l.value, l.obj_offset, false);
+    const auto parallel = [&](int count, auto&& f) {
+      std::atomic<int> next{0};
+      std::vector<std::thread> pool;
+      std::vector<std::string> errs(nth);
+      for (int t = 0; t < std::min(nth, count); ++t)
+        pool.emplace_back([&, t] {
+          try {
+            for (int b; (b = next.fetch_add(1)) < count;) f(b);
+          } catch (std::exception& e) {
+            errs[t] = e.what();
           }
-        } catch (std::exception& e) {
-          errs[t] = e.what();
-        }
-      });
-    for (auto& th : pool) th.join();
-    for (auto& e : errs)
-      if (!e.empty()) throw Error(B2P_ERR_INVALID, e);
+        });
+      for (auto& th : pool) th.join();
+      for (auto& e : errs)
+        if (!e.empty()) throw Error(B2P_ERR_INVALID, e);
+    };
+    parallel(ops, [&](int b) {
+      const b2p_lp& l = lps[b];
+      // structure and raw values; the scaling runs on the device below
+      P[b] = prepare_structure(l.num_rows, l.num_cols, l.start, l.index, l.value, l.obj_offset, false);
+    });
+    for (int b = ops; b < K; ++b) {
+      P[b].m = lps[b].num_rows;
+      P[b].n = lps[b].num_cols;
+      P[b].offset = lps[b].obj_offset;
+    }
+    inst_nnz.assign(K, 0);
+    for (int b = 0; b < K; ++b) inst_nnz[b] = static_cast<int64_t>(P[b < ops ? b : 0].A.val.size());
     stats.prepare_seconds = seconds_since(t0);
     // ---- block-diagonal concatenation ----
     roff.assign(K + 1, 0);
@@ -472,81 +496,35 @@ struct MultiEngine {
     for (int b = 0; b < K; ++b) {
       roff[b + 1] = roff[b] + P[b].m;
       coff[b + 1] = coff[b] + P[b].n;
-      annz += static_cast<int64_t>(P[b].A.val.size());
+      annz += inst_nnz[b];
     }
     if (roff[K] >= INT32_MAX || coff[K] >= INT32_MAX || annz >= INT32_MAX)
       throw Error(B2P_ERR_TOO_LARGE, "family exceeds 2^31 rows, columns or nonzeros");
     M = static_cast<int32_t>(roff[K]);
     N = static_cast<int32_t>(coff[K]);
+    Mo = static_cast<int32_t>(roff[ops]);
+    No = static_cast<int32_t>(coff[ops]);
     HostCsr A, AT;
-    A.rows = M;
-    A.cols = N;
-    AT.rows = N;
-    AT.cols = M;
-    std::vector<int64_t> aoff(K + 1, 0);  // first entry of LP b in the concatenated operators
-    for (int b = 0; b < K; ++b) aoff[b + 1] = aoff[b] + static_cast<int64_t>(P[b].A.val.size());
-    A.ptr.resize(static_cast<size_t>(M) + 1);
-    AT.ptr.resize(static_cast<size_t>(N) + 1);
+    A.rows = Mo;
+    A.cols = No;
+    AT.rows = No;
+    AT.cols = Mo;
+    std::vector<int64_t> aoff(ops + 1, 0);  // first entry of each operator in the concatenated ones
+    for (int b = 0; b < ops; ++b) aoff[b + 1] = aoff[b] + inst_nnz[b];
+    annz = aoff[ops];
+    A.ptr.resize(static_cast<size_t>(Mo) + 1);
+    AT.ptr.resize(static_cast<size_t>(No) + 1);
     A.ptr[0] = 0;
     AT.ptr[0] = 0;
-    std::vector<int32_t> rinst(M), cinst(N);
-    std::vector<double> rfac(M), cfac(N), c(N), lo(N), up(N), rl(M), ru(M), x0(N);
-    cNorm.assign(K, 0);
-    rhsNorm.assign(K, 0);
-    omega0.assign(K, 1.0);
     eta.assign(K, 0);
-    // every LP fills its own ranges: on all host threads, with the same values
-    // as one pass in LP order
-    auto parallel_lps = [&](auto&& f) {
-      std::atomic<int> nextb{0};
-      std::vector<std::thread> workers;
-      for (int t = 0; t < nth; ++t)
-        workers.emplace_back([&] {
-          for (int b; (b = nextb.fetch_add(1)) < K;) f(b);
-        });
-      for (auto& th : workers) th.join();
-    };
-    parallel_lps([&](int b) {
+    // every operator fills its own ranges: on all host threads, with the same
+    // values as one pass in order
+    parallel(ops, [&](int b) {
       const Prepared& p = P[b];
       const int32_t base = static_cast<int32_t>(aoff[b]);
       for (int32_t i = 0; i < p.m; ++i) A.ptr[roff[b] + i + 1] = base + p.A.ptr[i + 1];
       for (int32_t j = 0; j < p.n; ++j) AT.ptr[coff[b] + j + 1] = base + p.AT.ptr[j + 1];
     });
-    auto fill = [&](int b) {
-      const Prepared& p = P[b];
-      const b2p_lp& l = lps[b];
-      // scaled case vectors (src/pdhg/pdhg.cpp:466-481, 506-530), k = 1 per instance
-      double s = 0;
-      for (int32_t j = 0; j < p.n; ++j) s += l.col_cost[j] * l.col_cost[j];
-      cNorm[b] = std::sqrt(s);
-      s = 0;
-      for (int32_t i = 0; i < p.m; ++i) {
-        if (finite_bound(l.row_lower[i])) s += l.row_lower[i] * l.row_lower[i];
-        if (finite_bound(l.row_upper[i]) && l.row_upper[i] != l.row_lower[i]) s += l.row_upper[i] * l.row_upper[i];
-      }
-      rhsNorm[b] = std::sqrt(s);
-      double cn = 0, bn = 0;
-      for (int32_t j = 0; j < p.n; ++j) {
-        const size_t t = static_cast<size_t>(coff[b] + j);
-        cinst[t] = b;
-        cfac[t] = p.cfac[j];
-        c[t] = l.col_cost[j] * p.Cs[j] / p.gamma;
-        lo[t] = finite_bound(l.col_lower[j]) ? l.col_lower[j] / p.Cs[j] / p.beta : -HUGE_VAL;
-        up[t] = finite_bound(l.col_upper[j]) ? l.col_upper[j] / p.Cs[j] / p.beta : HUGE_VAL;
-        x0[t] = smin(smax(0.0, lo[t]), up[t]);
-        cn += c[t] * c[t];
-      }
-      for (int32_t i = 0; i < p.m; ++i) {
-        const size_t t = static_cast<size_t>(roff[b] + i);
-        rinst[t] = b;
-        rfac[t] = p.rfac[i];
-        rl[t] = finite_bound(l.row_lower[i]) ? l.row_lower[i] * p.R[i] / p.beta : -HUGE_VAL;
-        ru[t] = finite_bound(l.row_upper[i]) ? l.row_upper[i] * p.R[i] / p.beta : HUGE_VAL;
-        if (finite_bound(rl[t])) bn += rl[t] * rl[t];
-        if (finite_bound(ru[t]) && ru[t] != rl[t]) bn += ru[t] * ru[t];
-      }
-      if (cn > 1e-20 && bn > 1e-20) omega0[b] = std::sqrt(cn) / std::sqrt(bn);
-    };
     // ---- device ----
     const auto tx = Clock::now();
     dA_ptr = upload(A.ptr);
@@ -561,7 +539,7 @@ struct MultiEngine {
     B2P_CUDA(cudaMemsetAsync(dA_val + annz, 0, kTilePad * sizeof(double), stream));
     B2P_CUDA(cudaMemsetAsync(dT_idx + annz, 0, kTilePad * sizeof(int32_t), stream));
     B2P_CUDA(cudaMemsetAsync(dT_val + annz, 0, kTilePad * sizeof(double), stream));
-    for (int b = 0; b < K; ++b) {
+    for (int b = 0; b < ops; ++b) {
       const Prepared& p = P[b];
       const size_t e = p.A.val.size();
       if (!e) continue;
@@ -572,58 +550,48 @@ struct MultiEngine {
     }
     bytes_up += 24 * annz;
     {
-      std::vector<int32_t> co(K), ro(K);
-      for (int b = 0; b < K; ++b) {
-        co[b] = static_cast<int32_t>(coff[b]);
-        ro[b] = static_cast<int32_t>(roff[b]);
-      }
+      std::vector<int32_t> co(coff.begin(), coff.end()), ro(roff.begin(), roff.end());
       const int64_t* d_aoff = upload(aoff);
-      const int32_t* d_co = upload(co);
-      const int32_t* d_ro = upload(ro);
-      k_offset_segments<<<K, kBlock, 0, stream>>>(d_aoff, d_co, dA_idx);
-      k_offset_segments<<<K, kBlock, 0, stream>>>(d_aoff, d_ro, dT_idx);
-      B2P_CUDA(cudaGetLastError());
+      md.coff = upload(co);
+      md.roff = upload(ro);
+      if (ops > 1) {
+        k_offset_segments<<<ops, kBlock, 0, stream>>>(d_aoff, md.coff, dA_idx);
+        k_offset_segments<<<ops, kBlock, 0, stream>>>(d_aoff, md.roff, dT_idx);
+        B2P_CUDA(cudaGetLastError());
+      }
+      // co and ro go away; pageable copies are staged when the call returns
     }
     dT_ptr = upload(AT.ptr);
-    // ---- scaling on the device (Ruiz + Pock-Chambolle), rounding and the
-    // rescaling constants on the host, the scaled operators on the device ----
+    // ---- scaling on the device (Ruiz + Pock-Chambolle), rounding on the
+    // host, the scaled operators on the device ----
     const auto ts = Clock::now();
     {
-      std::vector<double> rs(M, 1.0), cs(N, 1.0);
+      std::vector<double> rs(Mo, 1.0), cs(No, 1.0);
       if (opt.ruiz_iterations > 0 && annz > 0)
         device_ruiz_factors(stream, device, viewA(), viewAT(), opt.ruiz_iterations, opt.pock_chambolle != 0, rs, cs);
-      const bool rescale = opt.rescale_objective_and_bounds != 0;
-      parallel_lps([&](int b) {
-        const b2p_lp& l = lps[b];
-        finish_scaling(P[b], rs.data() + roff[b], cs.data() + coff[b], l.col_cost, l.row_lower, l.row_upper,
-                       rescale);
-      });
-      std::vector<double> R(M), Cs(N);
-      for (int b = 0; b < K; ++b) {
+      std::vector<double> R(Mo), Cs(No);
+      parallel(ops, [&](int b) {
+        round_factors(P[b], rs.data() + roff[b], cs.data() + coff[b]);
         std::copy(P[b].R.begin(), P[b].R.end(), R.begin() + roff[b]);
         std::copy(P[b].Cs.begin(), P[b].Cs.end(), Cs.begin() + coff[b]);
-      }
+      });
+      md.R = upload(R);
+      md.Cs = upload(Cs);
       device_scale_operators(stream, device, viewA(), viewAT(), dA_val, dT_val, R, Cs);
     }
     stats.prepare_seconds += seconds_since(ts);
-    parallel_lps(fill);
-    d_rfac = upload(rfac);
-    d_cfac = upload(cfac);
+    for (int q = 0; q < MNSLOT; ++q) v[q] = dalloc<double>(q >= MY ? M : N);
+    std::vector<int32_t> rinst(one ? 0 : M, 0), cinst(No, 0);
+    if (!one)
+      parallel(K, [&](int b) {
+        std::fill(rinst.begin() + roff[b], rinst.begin() + roff[b + 1], b);
+        std::fill(cinst.begin() + coff[b], cinst.begin() + coff[b + 1], b);
+      });
     d_rinst = upload(rinst);
     d_cinst = upload(cinst);
+    setup_members(lps, parallel);
     device_power_iterations(40);
     for (int b = 0; b < K; ++b) eta[b] = 0.998 / P[b].normA;
-    for (int q = 0; q < MNSLOT; ++q) v[q] = dalloc<double>(q >= MY ? M : N);
-    auto put = [&](int q, const std::vector<double>& h) {
-      if (!h.empty()) B2P_CUDA(cudaMemcpyAsync(v[q], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-      bytes_up += static_cast<int64_t>(h.size() * sizeof(double));
-    };
-    put(MC, c);
-    put(MLO, lo);
-    put(MUP, up);
-    put(MRL, rl);
-    put(MRU, ru);
-    put(MXINIT, x0);
     if (M) B2P_CUDA(cudaMemsetAsync(v[MYINIT], 0, sizeof(double) * M, stream));
     d_tau = dalloc<double>(K);
     d_sigma = dalloc<double>(K);
@@ -631,12 +599,7 @@ struct MultiEngine {
     d_restart_at = dalloc<int64_t>(K);
     d_done = dalloc<int32_t>(K);
     d_mask = dalloc<int32_t>(K);
-    if (M > 0) {
-      k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), v[MXINIT], v[MAXINIT]);
-      B2P_CUDA(cudaGetLastError());
-    }
-    inst_nnz.assign(K, 0);
-    for (int b = 0; b < K; ++b) inst_nnz[b] = static_cast<int64_t>(P[b].A.val.size());
+    apply_a(v[MXINIT], v[MAXINIT]);
     cta = choose_cta();
     if (cta)
       setup_cta(A, AT);
@@ -647,6 +610,143 @@ struct MultiEngine {
     stats.setup_seconds = seconds_since(t0);
     stats.kernel_mode = B2P_KERNELS_FUSED;
     stats.precision_used = B2P_PRECISION_FP64;
+  }
+
+  // y = A x of every LP.
+  void apply_a(const double* x, double* y) {
+    if (M == 0) return;
+    if (ops == K)
+      k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), x, y);
+    else
+      k_member_spmv<<<blocks(M), kBlock, 0, stream>>>(M, P[0].m, P[0].n, viewA(), x, y);
+    B2P_CUDA(cudaGetLastError());
+  }
+
+  // Blocks along y for one thread per column and row of the largest LP.
+  unsigned member_blocks(bool cols, bool rows) const {
+    int32_t most = 1;
+    for (int b = 0; b < K; ++b) most = std::max(most, std::max(cols ? P[b].n : 0, rows ? P[b].m : 0));
+    return (most + kBlock - 1) / kBlock;
+  }
+
+  // The caller's costs, bounds and sides to the device (through a page-locked
+  // buffer filled by all host threads, up to kMemberStage; straight from the
+  // caller's arrays beyond), scaled there; the norms and rescaling constants
+  // back (pdhg_members.cuh).
+  static constexpr size_t kMemberStage = size_t(128) << 20;
+  template <class Parallel>
+  void setup_members(const b2p_lp* lps, Parallel&& parallel) {
+    const size_t nn = static_cast<size_t>(N), mm = static_cast<size_t>(M);
+    double* d_raw = dalloc<double>(3 * nn + 2 * mm);
+    md.cost = d_raw;
+    md.lower = d_raw + nn;
+    md.upper = d_raw + 2 * nn;
+    md.rl = d_raw + 3 * nn;
+    md.ru = d_raw + 3 * nn + mm;
+    md.shared = ops != K;
+    md.rescale = opt.rescale_objective_and_bounds != 0;
+    const size_t bytes = sizeof(double) * (3 * nn + 2 * mm);
+    bytes_up += static_cast<int64_t>(bytes);
+    // every array of LP b: its place in the concatenation, its length
+    const auto arrays = [&](int b, auto&& f) {
+      const b2p_lp& l = lps[b];
+      const size_t c0 = static_cast<size_t>(coff[b]), r0 = static_cast<size_t>(roff[b]);
+      f(c0, l.col_cost, P[b].n);
+      f(nn + c0, l.col_lower, P[b].n);
+      f(2 * nn + c0, l.col_upper, P[b].n);
+      f(3 * nn + r0, l.row_lower, P[b].m);
+      f(3 * nn + mm + r0, l.row_upper, P[b].m);
+    };
+    struct Stage {
+      double* p = nullptr;
+      size_t bytes = 0;
+      cudaStream_t stream;
+      ~Stage() {
+        if (!p) return;
+        cudaStreamSynchronize(stream);
+        PinnedCache::put(p, bytes);
+      }
+    } stage{nullptr, bytes, stream};
+    if (bytes > 0 && bytes <= kMemberStage) {
+      stage.p = static_cast<double*>(PinnedCache::get(bytes));
+      parallel(K, [&](int b) {
+        arrays(b, [&](size_t at, const double* src, int32_t len) {
+          if (len) std::memcpy(stage.p + at, src, sizeof(double) * len);
+        });
+      });
+      B2P_CUDA(cudaMemcpyAsync(d_raw, stage.p, bytes, cudaMemcpyHostToDevice, stream));
+    } else if (bytes > 0) {
+      for (int b = 0; b < K; ++b)
+        arrays(b, [&](size_t at, const double* src, int32_t len) {
+          if (len) B2P_CUDA(cudaMemcpyAsync(d_raw + at, src, sizeof(double) * len, cudaMemcpyHostToDevice, stream));
+        });
+    }
+    d_msums = dalloc<double>(static_cast<size_t>(K) * kMemberSums);
+    d_rfac = dalloc<double>(mm);
+    d_cfac = dalloc<double>(nn);
+    d_xans = dalloc<double>(nn);
+    d_yans = dalloc<double>(mm);
+    const unsigned k = static_cast<unsigned>(K);
+    k_member_raw_sums<<<dim3(k, 4), kOrderedThreads, 0, stream>>>(md, d_msums);
+    if (N)
+      k_member_columns<<<dim3(k, member_blocks(true, false)), kBlock, 0, stream>>>(md, d_msums, v[MC], v[MLO], v[MUP],
+                                                                                   v[MXINIT], d_cfac);
+    if (M)
+      k_member_rows<<<dim3(k, member_blocks(false, true)), kBlock, 0, stream>>>(md, d_msums, v[MRL], v[MRU], d_rfac);
+    k_member_scaled_sums<<<dim3(k, 2), kOrderedThreads, 0, stream>>>(md, v[MC], v[MRL], v[MRU], d_msums);
+    B2P_CUDA(cudaGetLastError());
+    std::vector<double> sums(static_cast<size_t>(K) * kMemberSums);
+    B2P_CUDA(cudaMemcpyAsync(sums.data(), d_msums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, stream));
+    B2P_CUDA(cudaStreamSynchronize(stream));
+    cNorm.assign(K, 0);
+    rhsNorm.assign(K, 0);
+    omega0.assign(K, 1.0);
+    for (int b = 0; b < K; ++b) {
+      const double* s = sums.data() + static_cast<size_t>(b) * kMemberSums;
+      P[b].gamma = md.rescale ? 1.0 + std::sqrt(s[MS_SC]) : 1.0;
+      P[b].beta = md.rescale ? 1.0 + std::sqrt(s[MS_SB]) : 1.0;
+      cNorm[b] = std::sqrt(s[MS_C]);
+      rhsNorm[b] = std::sqrt(s[MS_B]);
+      if (s[MS_RC] > 1e-20 && s[MS_RB] > 1e-20) omega0[b] = std::sqrt(s[MS_RC]) / std::sqrt(s[MS_RB]);
+    }
+  }
+
+  // x+ and y+ of LPs [first, first + count) into the answers.
+  void take_answers(int first, int count) {
+    if (count > 0 && (N || M))
+      k_member_answers<<<dim3(static_cast<unsigned>(count), member_blocks(true, true)), kBlock, 0, stream>>>(
+          md, first, d_msums, v[MXP], v[MYP], d_xans, d_yans);
+    B2P_CUDA(cudaGetLastError());
+  }
+
+  // The answers to the caller's arrays (NULL entries are skipped).
+  void fetch(double* const* x, double* const* y) {
+    const size_t nn = static_cast<size_t>(N), mm = static_cast<size_t>(M), bytes = sizeof(double) * (nn + mm);
+    if ((!x && !y) || bytes == 0) return;
+    const auto each = [&](auto&& f) {
+      for (int b = 0; b < K; ++b) {
+        if (x && x[b] && P[b].n) f(x[b], d_xans, static_cast<size_t>(coff[b]), size_t(0), P[b].n);
+        if (y && y[b] && P[b].m) f(y[b], d_yans, static_cast<size_t>(roff[b]), nn, P[b].m);
+      }
+    };
+    if (bytes > kMemberStage) {
+      each([&](double* dst, const double* src, size_t at, size_t, int32_t len) {
+        B2P_CUDA(cudaMemcpyAsync(dst, src + at, sizeof(double) * len, cudaMemcpyDeviceToHost, stream));
+      });
+      B2P_CUDA(cudaStreamSynchronize(stream));
+      return;
+    }
+    struct Stage {
+      double* p;
+      size_t bytes;
+      ~Stage() { PinnedCache::put(p, bytes); }
+    } stage{static_cast<double*>(PinnedCache::get(bytes)), bytes};
+    if (N) B2P_CUDA(cudaMemcpyAsync(stage.p, d_xans, sizeof(double) * nn, cudaMemcpyDeviceToHost, stream));
+    if (M) B2P_CUDA(cudaMemcpyAsync(stage.p + nn, d_yans, sizeof(double) * mm, cudaMemcpyDeviceToHost, stream));
+    B2P_CUDA(cudaStreamSynchronize(stream));
+    each([&](double* dst, const double*, size_t at, size_t base, int32_t len) {
+      std::memcpy(dst, stage.p + base + at, sizeof(double) * len);
+    });
   }
 
   // Whether all LPs have one A: equal sizes and equal column pointers, row
@@ -670,39 +770,31 @@ struct MultiEngine {
   // ||A|| of every LP on the device (1.01 x the power-iteration estimate, as
   // prepare() computes on the host), bit-identical to the host's.
   void device_power_iterations(int iters) {
-    if (M == 0 || N == 0) {
+    if (Mo == 0 || No == 0) {
       for (int b = 0; b < K; ++b) P[b].normA = 1.0 * 1.01;
       return;
     }
-    std::vector<int32_t> co(K + 1);
-    for (int b = 0; b <= K; ++b) co[b] = static_cast<int32_t>(coff[b]);
-    int32_t* d_co = upload(co);
-    int64_t* d_nnz = upload(inst_nnz_of_lps());
-    double* dx = dalloc<double>(N);
-    double* dy = dalloc<double>(M);
-    double* dz = dalloc<double>(N);
-    double* d_nz = dalloc<double>(K);
-    double* d_s = dalloc<double>(K);
-    int32_t* d_pdone = dalloc<int32_t>(K);
-    k_pi_init<<<blocks(std::max<int64_t>(N, K)), kBlock, 0, stream>>>(N, K, d_cinst, d_co, d_nnz, dx, d_pdone, d_s);
+    int64_t* d_nnz = upload(std::vector<int64_t>(inst_nnz.begin(), inst_nnz.begin() + ops));
+    double* dx = dalloc<double>(No);
+    double* dy = dalloc<double>(Mo);
+    double* dz = dalloc<double>(No);
+    double* d_nz = dalloc<double>(ops);
+    double* d_s = dalloc<double>(ops);
+    int32_t* d_pdone = dalloc<int32_t>(ops);
+    k_pi_init<<<blocks(std::max<int64_t>(No, ops)), kBlock, 0, stream>>>(No, ops, d_cinst, md.coff, d_nnz, dx, d_pdone,
+                                                                        d_s);
     for (int it = 0; it < iters; ++it) {
-      k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), dx, dy);
-      k_spmv<<<blocks(N), kBlock, 0, stream>>>(N, 1, viewAT(), dy, dz);
-      k_pi_norm<<<K, kOrderedThreads, 0, stream>>>(d_co, dz, d_pdone, d_nz, d_s);
-      k_pi_scale<<<blocks(N), kBlock, 0, stream>>>(N, d_cinst, d_pdone, d_nz, dz, dx);
+      k_spmv<<<blocks(Mo), kBlock, 0, stream>>>(Mo, 1, viewA(), dx, dy);
+      k_spmv<<<blocks(No), kBlock, 0, stream>>>(No, 1, viewAT(), dy, dz);
+      k_pi_norm<<<ops, kOrderedThreads, 0, stream>>>(md.coff, dz, d_pdone, d_nz, d_s);
+      k_pi_scale<<<blocks(No), kBlock, 0, stream>>>(No, d_cinst, d_pdone, d_nz, dz, dx);
     }
     B2P_CUDA(cudaGetLastError());
-    std::vector<double> s(K);
-    B2P_CUDA(cudaMemcpyAsync(s.data(), d_s, sizeof(double) * K, cudaMemcpyDeviceToHost, stream));
+    std::vector<double> s(ops);
+    B2P_CUDA(cudaMemcpyAsync(s.data(), d_s, sizeof(double) * ops, cudaMemcpyDeviceToHost, stream));
     B2P_CUDA(cudaStreamSynchronize(stream));
-    for (int b = 0; b < K; ++b) P[b].normA = s[b] * 1.01;
+    for (int b = 0; b < K; ++b) P[b].normA = s[b < ops ? b : 0] * 1.01;
   }
-  std::vector<int64_t> inst_nnz_of_lps() const {
-    std::vector<int64_t> v(K);
-    for (int b = 0; b < K; ++b) v[b] = static_cast<int64_t>(P[b].A.val.size());
-    return v;
-  }
-
   // Block-diagonal form: check tables, fused-kernel schedules, autotuner.
   void setup_grid(const HostCsr& A, const HostCsr& AT, int64_t annz) {
     stats.multi_form = B2P_MULTI_GRID;
@@ -778,7 +870,7 @@ struct MultiEngine {
   }
   int cta_tier(int b, int64_t budget, int esize = 8) const {
     const Prepared& p = P[b];
-    const int64_t nnz = static_cast<int64_t>(p.A.val.size());
+    const int64_t nnz = inst_nnz[b];
     if (cta_tier_bytes(kCtaAll, p.m, p.n, nnz, esize) <= budget) return kCtaAll;
     if (cta_tier_bytes(kCtaVectorsPtr, p.m, p.n, nnz, esize) <= budget) return kCtaVectorsPtr;
     if (cta_tier_bytes(kCtaVectors, p.m, p.n, nnz, esize) <= budget) return kCtaVectors;
@@ -819,7 +911,7 @@ struct MultiEngine {
         c.aptr_off = c.tshift = static_cast<int32_t>(roff[b]);
         c.tptr_off = c.ashift = static_cast<int32_t>(coff[b]);
       }
-      c.nnz = static_cast<int32_t>(p.A.val.size());
+      c.nnz = static_cast<int32_t>(inst_nnz[b]);
       c.tier = cta_tier(b, budget);
       c.tier32 = cta_tier(b, budget, 4);
       c.pad = 0;
@@ -878,7 +970,7 @@ struct MultiEngine {
   // slice + 32 q + l.  Not built when the padded copy would exceed 2^31
   // entries.
   void build_sliced(const HostCsr& A, const HostCsr& AT) {
-    const int nlp = shared_operator ? std::min(K, 1) : K;
+    const int nlp = ops;
     auto bases = [&](const HostCsr& H, const std::vector<int64_t>& off, bool cols, std::vector<int32_t>& base,
                      int64_t& total) {
       base.assign(H.ptr.size() > 0 ? H.ptr.size() - 1 : 0, 0);
@@ -911,7 +1003,7 @@ struct MultiEngine {
     B2P_CUDA(cudaMemsetAsync(d_sa_val, 0, sizeof(double) * std::max<int64_t>(sa_len, 1), stream));
     B2P_CUDA(cudaMemsetAsync(d_st_idx, 0, sizeof(int32_t) * std::max<int64_t>(st_len, 1), stream));
     B2P_CUDA(cudaMemsetAsync(d_st_val, 0, sizeof(double) * std::max<int64_t>(st_len, 1), stream));
-    const int32_t ra = nlp == K ? M : P[0].m, rt = nlp == K ? N : P[0].n;
+    const int32_t ra = Mo, rt = No;
     if (ra) k_to_sliced<<<blocks(ra), kBlock, 0, stream>>>(ra, dA_ptr, dA_idx, dA_val, d_sa_base, d_sa_idx, d_sa_val);
     if (rt) k_to_sliced<<<blocks(rt), kBlock, 0, stream>>>(rt, dT_ptr, dT_idx, dT_val, d_st_base, d_st_idx, d_st_val);
     B2P_CUDA(cudaGetLastError());
@@ -950,7 +1042,8 @@ struct MultiEngine {
   // FP32 run of the mixed form: FP32 copies of the scaled operators' values,
   // FP32 global-tier state, the FP64 run's starting point, kernel attributes.
   void setup_cta_fp32() {
-    const size_t annz = static_cast<size_t>(inst_nnz_total());
+    size_t annz = 0;
+    for (int b = 0; b < ops; ++b) annz += static_cast<size_t>(inst_nnz[b]);
     dA_val32 = dalloc<float>(annz);
     dT_val32 = dalloc<float>(annz);
     if (annz) {
@@ -1174,8 +1267,6 @@ struct MultiEngine {
     const auto t_solve = Clock::now();
     results.assign(K, b2p_result{});
     weights.assign(K, 1.0);
-    xs.assign(K, {});
-    ys.assign(K, {});
     *reinterpret_cast<volatile int32_t*>(h_stop) = 0;
     bool raised = false;
     auto wait_for = [&](cudaEvent_t ev) {
@@ -1239,7 +1330,7 @@ struct MultiEngine {
         if (N) k_clamp_to_bounds<<<blocks(N), kBlock, 0, stream>>>(N, v[MXP], v[MLO], v[MUP], d_x2);
         if (M) {
           B2P_CUDA(cudaMemcpyAsync(d_y2, v[MYP], sizeof(double) * M, cudaMemcpyDeviceToDevice, stream));
-          k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), d_x2, d_ax2);
+          apply_a(d_x2, d_ax2);
         }
         B2P_CUDA(cudaGetLastError());
         CtaArgs a2 = cta_args(opt.tolerance, opt.max_iterations);
@@ -1258,10 +1349,8 @@ struct MultiEngine {
     float ms = 0;
     B2P_CUDA(cudaEventElapsedTime(&ms, ev_start, ev_stop));
     stats.kernel_seconds = ms / 1000.0;
-    std::vector<double> xp(N), yp(M);
+    take_answers(0, K);
     B2P_CUDA(cudaMemcpyAsync(out.data(), d_out, sizeof(CtaOut) * K, cudaMemcpyDeviceToHost, stream));
-    if (N) B2P_CUDA(cudaMemcpyAsync(xp.data(), v[MXP], sizeof(double) * N, cudaMemcpyDeviceToHost, stream));
-    if (M) B2P_CUDA(cudaMemcpyAsync(yp.data(), v[MYP], sizeof(double) * M, cudaMemcpyDeviceToHost, stream));
     B2P_CUDA(cudaStreamSynchronize(stream));
     bytes_down += static_cast<int64_t>(sizeof(CtaOut) * K + sizeof(double) * (static_cast<int64_t>(N) + M));
     int64_t its = 0, its32 = 0;
@@ -1276,7 +1365,7 @@ struct MultiEngine {
         its32 = std::max<int64_t>(its32, out32[b].iterations);
         if (o.status == kCtaStalled) o.status = B2P_STATUS_ITERATION_LIMIT;
       }
-      store_result(b, o.status, o.rel_kkt, o.pobj, o.dobj, o.iterations, xp.data() + coff[b], yp.data() + roff[b]);
+      store_result(b, o.status, o.rel_kkt, o.pobj, o.dobj, o.iterations);
       weights[b] = o.omega * P[b].gamma / P[b].beta;
       its = std::max<int64_t>(its, o.iterations + (o.status == B2P_STATUS_OPTIMAL ? 1 : 0));
       stats.restarts += o.restarts;
@@ -1317,19 +1406,19 @@ struct MultiEngine {
     B2P_CUDA(cudaStreamSynchronize(stream));
     for (int b = 0; b < K; ++b) {
       const Prepared& p = P[b];
+      const Prepared& f = P[b < ops ? b : 0];  // the operator's factors
       if (xst && xst[b])
         for (int32_t j = 0; j < p.n; ++j) {
           const size_t t = static_cast<size_t>(coff[b] + j);
-          x0[t] = smin(smax(xst[b][j] / p.Cs[j] / p.beta, lo[t]), up[t]);
+          x0[t] = smin(smax(xst[b][j] / f.Cs[j] / p.beta, lo[t]), up[t]);
         }
       if (yst && yst[b])
-        for (int32_t i = 0; i < p.m; ++i) y0[static_cast<size_t>(roff[b] + i)] = yst[b][i] / p.R[i] / p.gamma;
+        for (int32_t i = 0; i < p.m; ++i) y0[static_cast<size_t>(roff[b] + i)] = yst[b][i] / f.R[i] / p.gamma;
     }
     if (N) B2P_CUDA(cudaMemcpyAsync(v[MXINIT], x0.data(), sizeof(double) * N, cudaMemcpyHostToDevice, stream));
     if (M) {
       B2P_CUDA(cudaMemcpyAsync(v[MYINIT], y0.data(), sizeof(double) * M, cudaMemcpyHostToDevice, stream));
-      k_spmv<<<blocks(M), kBlock, 0, stream>>>(M, 1, viewA(), v[MXINIT], v[MAXINIT]);
-      B2P_CUDA(cudaGetLastError());
+      apply_a(v[MXINIT], v[MAXINIT]);
     }
     B2P_CUDA(cudaStreamSynchronize(stream));
   }
@@ -1729,25 +1818,13 @@ struct MultiEngine {
   }
 
   void extract(int b, int status, double relKkt, double pobj, double dobj, int64_t it) {
-    const Prepared& p = P[b];
-    std::vector<double> xp(p.n), yp(p.m);
-    if (p.n)
-      B2P_CUDA(cudaMemcpyAsync(xp.data(), v[MXP] + coff[b], sizeof(double) * p.n, cudaMemcpyDeviceToHost, stream));
-    if (p.m)
-      B2P_CUDA(cudaMemcpyAsync(yp.data(), v[MYP] + roff[b], sizeof(double) * p.m, cudaMemcpyDeviceToHost, stream));
-    B2P_CUDA(cudaStreamSynchronize(stream));
-    bytes_down += static_cast<int64_t>(sizeof(double) * (p.n + p.m));
-    store_result(b, status, relKkt, pobj, dobj, it, xp.data(), yp.data());
+    take_answers(b, 1);
+    bytes_down += static_cast<int64_t>(sizeof(double) * (P[b].n + P[b].m));
+    store_result(b, status, relKkt, pobj, dobj, it);
   }
 
-  // Unscaled answer of instance b from its scaled x+ and y+ (src/pdhg/pdhg.cpp:668-680).
-  void store_result(int b, int status, double relKkt, double pobj, double dobj, int64_t it, const double* xp,
-                    const double* yp) {
+  void store_result(int b, int status, double relKkt, double pobj, double dobj, int64_t it) {
     const Prepared& p = P[b];
-    xs[b].resize(p.n);
-    ys[b].resize(p.m);
-    for (int32_t j = 0; j < p.n; ++j) xs[b][j] = xp[j] * p.Cs[j] * p.beta;
-    for (int32_t i = 0; i < p.m; ++i) ys[b][i] = yp[i] * p.R[i] * p.gamma;
     b2p_result& r = results[b];
     r.status = status;
     r.iterations = it;
@@ -1769,8 +1846,6 @@ struct MultiEngine {
     std::vector<double> omega = omega0;
     results.assign(K, b2p_result{});
     weights.assign(K, 1.0);
-    xs.assign(K, {});
-    ys.assign(K, {});
     stats.restarts = 0;
     std::vector<char> done(K, 0);
     std::vector<RestartTracker> restarts(K);
@@ -1876,10 +1951,8 @@ extern "C" int b2p_solve_pdhg_multi_warm(const b2p_lp* lps, int32_t num_lps, con
     e.create(lps, num_lps, opts);
     e.set_start(x_start, row_dual_start, primal_weight_start);
     e.solve(t0);
+    e.fetch(x, row_dual);
     for (int b = 0; b < e.K; ++b) {
-      if (x && x[b] && !e.xs[b].empty()) std::memcpy(x[b], e.xs[b].data(), sizeof(double) * e.xs[b].size());
-      if (row_dual && row_dual[b] && !e.ys[b].empty())
-        std::memcpy(row_dual[b], e.ys[b].data(), sizeof(double) * e.ys[b].size());
       if (primal_weight) primal_weight[b] = e.weights[b];
       if (results) results[b] = e.results[b];
     }

@@ -289,11 +289,15 @@ Prepared prepare_structure(int32_t m, int32_t n, const int32_t* start, const int
   return P;
 }
 
+void round_factors(Prepared& P, const double* rs, const double* cs) {
+  for (int32_t i = 0; i < P.m; ++i) P.R[i] = pow2_round(rs[i]);
+  for (int32_t j = 0; j < P.n; ++j) P.Cs[j] = pow2_round(cs[j]);
+}
+
 void finish_scaling(Prepared& P, const double* rs, const double* cs, const double* cost, const double* row_lower,
                     const double* row_upper, bool rescale) {
   const int32_t m = P.m, n = P.n;
-  for (int32_t i = 0; i < m; ++i) P.R[i] = pow2_round(rs[i]);
-  for (int32_t j = 0; j < n; ++j) P.Cs[j] = pow2_round(cs[j]);
+  round_factors(P, rs, cs);
   P.beta = P.gamma = 1.0;
   if (rescale) {
     double cn = 0, bn = 0;

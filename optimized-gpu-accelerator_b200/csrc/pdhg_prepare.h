@@ -61,6 +61,9 @@ Prepared prepare_structure(int32_t m, int32_t n, const int32_t* start, const int
 void finish_scaling(Prepared& P, const double* rs, const double* cs, const double* cost, const double* row_lower,
                     const double* row_upper, bool rescale);
 
+// Its first part: R and Cs, the factors' power-of-two rounding.
+void round_factors(Prepared& P, const double* rs, const double* cs);
+
 double pow2_round(double v);
 
 double power_iteration(int32_t m, int32_t n, const int32_t* start, const int32_t* index, const double* value,

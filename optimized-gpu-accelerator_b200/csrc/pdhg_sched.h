@@ -15,17 +15,21 @@
 
 namespace b2p {
 
-inline void check_lp(const b2p_lp* lp) {
+// `structure`: the column pointers and row indices too (false for an LP that
+// has another, already checked one's arrays).
+inline void check_lp(const b2p_lp* lp, bool structure = true) {
   if (!lp) throw Error(B2P_ERR_INVALID, "lp is NULL");
   if (lp->num_rows < 0 || lp->num_cols < 0) throw Error(B2P_ERR_INVALID, "negative dimension");
-  if (!lp->start) throw Error(B2P_ERR_INVALID, "start is NULL");
-  if (lp->start[0] != 0) throw Error(B2P_ERR_INVALID, "start[0] must be 0");
-  for (int32_t j = 0; j < lp->num_cols; ++j)
-    if (lp->start[j + 1] < lp->start[j]) throw Error(B2P_ERR_INVALID, "start must be non-decreasing");
-  const int32_t nnz = lp->start[lp->num_cols];
-  if (nnz > 0 && (!lp->index || !lp->value)) throw Error(B2P_ERR_INVALID, "index/value are NULL");
-  for (int32_t q = 0; q < nnz; ++q)
-    if (lp->index[q] < 0 || lp->index[q] >= lp->num_rows) throw Error(B2P_ERR_INVALID, "row index out of range");
+  if (structure) {
+    if (!lp->start) throw Error(B2P_ERR_INVALID, "start is NULL");
+    if (lp->start[0] != 0) throw Error(B2P_ERR_INVALID, "start[0] must be 0");
+    for (int32_t j = 0; j < lp->num_cols; ++j)
+      if (lp->start[j + 1] < lp->start[j]) throw Error(B2P_ERR_INVALID, "start must be non-decreasing");
+    const int32_t nnz = lp->start[lp->num_cols];
+    if (nnz > 0 && (!lp->index || !lp->value)) throw Error(B2P_ERR_INVALID, "index/value are NULL");
+    for (int32_t q = 0; q < nnz; ++q)
+      if (lp->index[q] < 0 || lp->index[q] >= lp->num_rows) throw Error(B2P_ERR_INVALID, "row index out of range");
+  }
   if (lp->num_cols > 0 && (!lp->col_cost || !lp->col_lower || !lp->col_upper))
     throw Error(B2P_ERR_INVALID, "column vectors are NULL");
   if (lp->num_rows > 0 && (!lp->row_lower || !lp->row_upper)) throw Error(B2P_ERR_INVALID, "row vectors are NULL");
