@@ -383,7 +383,7 @@ struct Engine {
       int sms = 0;
       B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
       const int64_t wave = static_cast<int64_t>(std::max(1, per_sm)) * sms * kBlock;
-      const int rounds = opt.short_row_rounds > 0 ? opt.short_row_rounds : 2;
+      const int rounds = std::max(0, opt.short_row_rounds);
       binsA = device_bins(P.A, wave, opt.lanes_per_row_a, rounds);
       binsT = device_bins(P.AT, wave, opt.lanes_per_row_at, rounds);
       stats.lanes_per_row_a = binsA.g;

@@ -344,7 +344,7 @@ struct MultiEngine {
   int64_t sched_nnz = 0;
   int ltA = 0, ltT = 0;
   int64_t wave = 0;
-  int rounds = 2;
+  int rounds = 0;
   // Per operator, when chosen: the warp-tile schedule of the short rows plus a
   // binned schedule of the long rows only (pdhg_tiled.cuh).
   struct TileSched {
@@ -828,7 +828,7 @@ struct MultiEngine {
     B2P_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dual_binned<4, true, true>, kBlock, 0));
     B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     wave = static_cast<int64_t>(std::max(1, per_sm)) * sms * kBlock;
-    rounds = opt.short_row_rounds > 0 ? opt.short_row_rounds : 2;
+    rounds = std::max(0, opt.short_row_rounds);
     const HostBins hbA = make_bins(A, wave, opt.lanes_per_row_a, rounds);
     const HostBins hbT = make_bins(AT, wave, opt.lanes_per_row_at, rounds);
     binsA = device_bins(hbA, M);

@@ -42,12 +42,21 @@ struct HostBins {
   int long_thr = kUnroll;
 };
 
-// Lanes per short row: enough that 90% of the rows finish in one round of
-// kUnroll entries per lane; when fewer lanes would let the whole grid fit in
-// one wave of `wave_threads` (a latency-bound operator), the most that fit.
-// Operators too large for one wave keep the row-length choice (their waves
-// pipeline and the kernels are bandwidth-bound).  `rounds` rounds of kUnroll
-// entries stay on the short path.
+// Lanes per short row.  An operator whose rows fit one wave of `wave_threads`
+// is bound by latency: enough lanes that 90% of the rows finish in one round
+// of kUnroll entries per lane, or the most that keep the grid in one wave.  A
+// larger one is bound by what its warps issue: lanes without an entry cost as
+// much as the others, so the fewest that take 90% of the rows in three rounds
+// (transportation LP of 2 M nonzeros, A's rows of 8 +- 3 entries, us per dual
+// launch with 8 / 4 / 2 / 1 lanes: 37.0 / 24.9 / 20.8 / 20.4).
+// `rounds` rounds of kUnroll entries stay on the short path; 0: two, unless
+// the rows beyond those -- a warp each -- would fill a quarter of a wave, then
+// four, and rows of up to kShortRow entries whatever the lanes (us per
+// iteration with two rounds / so: transportation LPs of 2 M nonzeros, one lane,
+// 72.8 / 29.5, of 1 M 32.1 / 16.1, random LP of 1.2 M 43.4 / 19.4, 24 uneven
+// LPs with two lanes 27.0 / 23.8; a 15,000 x 21,000 plan with few such rows,
+// which then wait for one lane, 4.8 / 7.5).
+constexpr int kShortRow = 24;
 inline HostBins make_bins(const HostCsr& M, int64_t wave_threads, int g_override, int rounds) {
   HostBins hb;
   std::vector<int32_t> len(M.rows);
@@ -59,11 +68,19 @@ inline HostBins make_bins(const HostCsr& M, int64_t wave_threads, int g_override
     const size_t q = static_cast<size_t>(0.9 * (sorted.size() - 1));
     std::nth_element(sorted.begin(), sorted.begin() + q, sorted.end());
     const int p90 = sorted[q];
-    while (hb.g < 32 && hb.g * kUnroll < p90) hb.g *= 2;
-    if (static_cast<int64_t>(M.rows) <= wave_threads)
+    if (static_cast<int64_t>(M.rows) <= wave_threads) {
+      while (hb.g < 32 && hb.g * kUnroll < p90) hb.g *= 2;
       while (hb.g > 1 && static_cast<int64_t>(M.rows) * hb.g > wave_threads) hb.g /= 2;
+    } else {
+      while (hb.g < 32 && 3 * hb.g * kUnroll < p90) hb.g *= 2;
+    }
   }
-  hb.long_thr = std::max(1, rounds) * kUnroll * hb.g;
+  hb.long_thr = (rounds > 0 ? rounds : 2) * kUnroll * hb.g;
+  if (rounds <= 0) {
+    int64_t beyond = 0;
+    for (int32_t l : len) beyond += l > hb.long_thr && l <= kVeryLongRow;
+    if (beyond * 32 * 4 > wave_threads) hb.long_thr = std::max(4 * kUnroll * hb.g, kShortRow);
+  }
   for (int32_t i = 0; i < M.rows; ++i) {
     if (len[i] > kVeryLongRow)
       hb.vlong_rows.push_back(i);
