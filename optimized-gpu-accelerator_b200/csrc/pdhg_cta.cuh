@@ -112,7 +112,7 @@ struct CtaArgs {
   int32_t entry_check;   // measure the starting point first; stop there if it meets tol
   int32_t stall_checks;  // > 0: end the run after this many checks without a 10% KKT gain
   int32_t pad;
-  const volatile int32_t* stop;  // host-mapped; nonzero = stop at the next check
+  const volatile int32_t* stop;  // device word; nonzero = stop at the next check (NULL: nothing stops the run)
 };
 
 template <class T>
@@ -171,9 +171,14 @@ struct Ctl {
   int32_t pad;
 };
 
-template <int NT>
+// A check's sums have one order whatever the variant, so that a solve does not
+// depend on which one the autotuner found fastest: kSumThreads virtual
+// threads, virtual thread v adding the elements v, v + kSumThreads, ..., a
+// shuffle tree over each 32 of them, then those warps in order.  A block of
+// NT threads plays them in kSumThreads / NT passes.
+constexpr int kSumThreads = 1024;
 struct Shared {
-  double w[kNumSums][NT / 32];
+  double w[kNumSums][kSumThreads / 32];
   double tot[kNumSums];
   Ctl ctl;
 };
@@ -254,30 +259,38 @@ __device__ __noinline__ void decide(Ctl& c, const double* tot, double scale_obj,
   }
 }
 
-// Block sums of s in a fixed order, then the decisions; on return every
-// thread sees sh.ctl of this check.  `it` = index of the check iteration.
+// Warp sums of pass `pass` into their place.
 template <int NT>
-__device__ __forceinline__ void check_decide(double (&s)[kNumSums], Shared<NT>& sh, const CtaArgs& a,
-                                             const CtaLp& L, int64_t it) {
+__device__ __forceinline__ void pass_sums(double (&s)[kNumSums], Shared& sh, int pass) {
 #pragma unroll
   for (int q = 0; q < kNumSums; ++q)
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
+  if ((threadIdx.x & 31) == 0)
 #pragma unroll
-    for (int q = 0; q < kNumSums; ++q) sh.w[q][warp] = s[q];
+    for (int q = 0; q < kNumSums; ++q) sh.w[q][pass * (NT / 32) + (threadIdx.x >> 5)] = s[q];
+}
+
+// The virtual warps in order; lanes of one warp (the result is lane q's).
+__device__ __forceinline__ void total_sums(Shared& sh) {
+  const int lane = threadIdx.x & 31;
+  if (lane < kNumSums) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int w = 0; w < kSumThreads / 32; ++w) t += sh.w[lane][w];
+    sh.tot[lane] = t;
+  }
+  __syncwarp();
+}
+
+// After every pass_sums: the totals, then the decisions; on return every
+// thread sees sh.ctl of this check.  `it` = index of the check iteration.
+__device__ __forceinline__ void check_decide(Shared& sh, const CtaArgs& a, const CtaLp& L, int64_t it) {
   if (threadIdx.x == 0) sh.ctl.stop = a.stop ? *a.stop : 0;
   __syncthreads();
-  if (warp == 0) {
-    if (lane < kNumSums) {
-      double t = 0.0;
-#pragma unroll
-      for (int w = 0; w < NT / 32; ++w) t += sh.w[lane][w];
-      sh.tot[lane] = t;
-    }
-    __syncwarp();
-    if (lane == 0)
+  if (threadIdx.x < 32) {
+    total_sums(sh);
+    if (threadIdx.x == 0)
       decide(sh.ctl, sh.tot, L.scale_obj, L.rhsnorm, L.cnorm, L.eta, it, a.tol, a.check_every, a.stall_checks);
   }
   __syncthreads();
@@ -285,27 +298,11 @@ __device__ __forceinline__ void check_decide(double (&s)[kNumSums], Shared<NT>& 
 
 // The termination test alone, on sums of the starting point (entry check):
 // on return every thread sees sh.ctl.status.
-template <int NT>
-__device__ __forceinline__ void entry_decide(double (&s)[kNumSums], Shared<NT>& sh, const CtaArgs& a,
-                                             const CtaLp& L) {
-#pragma unroll
-  for (int q = 0; q < kNumSums; ++q)
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < kNumSums; ++q) sh.w[q][warp] = s[q];
+__device__ __forceinline__ void entry_decide(Shared& sh, const CtaArgs& a, const CtaLp& L) {
   __syncthreads();
-  if (warp == 0) {
-    if (lane < kNumSums) {
-      double t = 0.0;
-#pragma unroll
-      for (int w = 0; w < NT / 32; ++w) t += sh.w[lane][w];
-      sh.tot[lane] = t;
-    }
-    __syncwarp();
-    if (lane == 0) {
+  if (threadIdx.x < 32) {
+    total_sums(sh);
+    if (threadIdx.x == 0) {
       Ctl& c = sh.ctl;
       const double* tot = sh.tot;
       c.pobj = tot[CS_POBJ] * L.scale_obj;
@@ -319,7 +316,6 @@ __device__ __forceinline__ void entry_decide(double (&s)[kNumSums], Shared<NT>& 
   __syncthreads();
 }
 
-template <int NT>
 __device__ __forceinline__ void write_out(const CtaArgs& a, const Ctl& c, int lp, int64_t it) {
   if (threadIdx.x != 0) return;
   CtaOut o;
@@ -433,7 +429,7 @@ __device__ __forceinline__ void col_check(double (&s)[kNumSums], double atyp, do
 
 template <int NT, int TIER, class T>
 __device__ __forceinline__ void run_lp(const CtaArgs& a, const CtaLp& L, int lp, unsigned char* smem,
-                                       Shared<NT>& sh) {
+                                       Shared& sh) {
   const int m = L.m, n = L.n, tid = threadIdx.x;
   const CtaState<T> g = cta_state(a, static_cast<T*>(nullptr));
   T *x, *xp, *x0, *y, *yp, *y0, *ax, *axp, *ax0;
@@ -507,19 +503,22 @@ __device__ __forceinline__ void run_lp(const CtaArgs& a, const CtaLp& L, int lp,
   int64_t restartAt = L.it0, it = L.it0;
   if (a.entry_check) {
     // the starting point measured as it is (x+ = x, y+ = y, A x+ = A x)
-    double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = tid; i < m; i += NT) {
-      const double yv = static_cast<double>(y[i]);
-      row_check(s, static_cast<double>(ax[i]), rl[i], ru[i], rfac[i], yv, yv, yv);
-      axp[i] = ax[i];
-      yp[i] = y[i];
+    for (int pass = 0; pass < kSumThreads / NT; ++pass) {
+      double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+      for (int i = tid + pass * NT; i < m; i += kSumThreads) {
+        const double yv = static_cast<double>(y[i]);
+        row_check(s, static_cast<double>(ax[i]), rl[i], ru[i], rfac[i], yv, yv, yv);
+        axp[i] = ax[i];
+        yp[i] = y[i];
+      }
+      for (int j = tid + pass * NT; j < n; j += kSumThreads) {
+        const double xv = static_cast<double>(x[j]);
+        col_check(s, opT.sum(j, y), c[j], lo[j], up[j], cfac[j], xv, xv, xv);
+        xp[j] = x[j];
+      }
+      pass_sums<NT>(s, sh, pass);
     }
-    for (int j = tid; j < n; j += NT) {
-      const double xv = static_cast<double>(x[j]);
-      col_check(s, opT.sum(j, y), c[j], lo[j], up[j], cfac[j], xv, xv, xv);
-      xp[j] = x[j];
-    }
-    entry_decide<NT>(s, sh, a, L);
+    entry_decide(sh, a, L);
     if (sh.ctl.status) it = L.it0 - 1;  // reported as the check iteration that produced the point
   }
   while (!sh.ctl.status && it < a.max_it) {
@@ -561,22 +560,26 @@ __device__ __forceinline__ void run_lp(const CtaArgs& a, const CtaLp& L, int lp,
     // ---- check at iteration it + Lint - 1, then the deferred Halpern step of
     // that iteration on the same elements
     const double lam = lambda_at(it + Lint - 1 - restartAt);
-    double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = tid; i < m; i += NT) {
-      const double yc = static_cast<double>(y[i]), yv = static_cast<double>(yp[i]);
-      const double y0v = static_cast<double>(y0[i]), axpv = static_cast<double>(axp[i]);
-      row_check(s, axpv, rl[i], ru[i], rfac[i], yv, yc, y0v);
-      y[i] = static_cast<T>(halpern_step(yc, yv, y0v, lam, rho));
-      ax[i] = static_cast<T>(halpern_step(static_cast<double>(ax[i]), axpv, static_cast<double>(ax0[i]), lam, rho));
-    }
-    for (int j = tid; j < n; j += NT) {
-      const double atyp = opT.sum(j, yp);
-      const double xc = static_cast<double>(x[j]), xpv = static_cast<double>(xp[j]), x0v = static_cast<double>(x0[j]);
-      col_check(s, atyp, c[j], lo[j], up[j], cfac[j], xpv, xc, x0v);
-      x[j] = static_cast<T>(halpern_step(xc, xpv, x0v, lam, rho));
+    for (int pass = 0; pass < kSumThreads / NT; ++pass) {
+      double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+      for (int i = tid + pass * NT; i < m; i += kSumThreads) {
+        const double yc = static_cast<double>(y[i]), yv = static_cast<double>(yp[i]);
+        const double y0v = static_cast<double>(y0[i]), axpv = static_cast<double>(axp[i]);
+        row_check(s, axpv, rl[i], ru[i], rfac[i], yv, yc, y0v);
+        y[i] = static_cast<T>(halpern_step(yc, yv, y0v, lam, rho));
+        ax[i] = static_cast<T>(halpern_step(static_cast<double>(ax[i]), axpv, static_cast<double>(ax0[i]), lam, rho));
+      }
+      for (int j = tid + pass * NT; j < n; j += kSumThreads) {
+        const double atyp = opT.sum(j, yp);
+        const double xc = static_cast<double>(x[j]), xpv = static_cast<double>(xp[j]);
+        const double x0v = static_cast<double>(x0[j]);
+        col_check(s, atyp, c[j], lo[j], up[j], cfac[j], xpv, xc, x0v);
+        x[j] = static_cast<T>(halpern_step(xc, xpv, x0v, lam, rho));
+      }
+      pass_sums<NT>(s, sh, pass);
     }
     it += Lint - 1;
-    check_decide<NT>(s, sh, a, L, it);
+    check_decide(sh, a, L, it);
     if (sh.ctl.status) break;
     if (sh.ctl.restart) {
       tau = sh.ctl.tau;
@@ -596,7 +599,7 @@ __device__ __forceinline__ void run_lp(const CtaArgs& a, const CtaLp& L, int lp,
     for (int j = tid; j < n; j += NT) a.xp[L.coff + j] = static_cast<double>(xp[j]);
     for (int i = tid; i < m; i += NT) a.yp[L.roff + i] = static_cast<double>(yp[i]);
   }
-  write_out<NT>(a, sh.ctl, lp, it);
+  write_out(a, sh.ctl, lp, it);
 }
 
 // Owner variant: for LPs with max(m, n) <= R * NT and both operators in
@@ -607,7 +610,7 @@ __device__ __forceinline__ void run_lp(const CtaArgs& a, const CtaLp& L, int lp,
 // vectors other threads gather (x+, y, and y+ at check iterations).
 template <int NT, int R>
 __device__ __forceinline__ void run_owner(const CtaArgs& a, const CtaLp& L, int lp, unsigned char* smem,
-                                          Shared<NT>& sh) {
+                                          Shared& sh) {
   const int m = L.m, n = L.n, tid = threadIdx.x;
   double* xp_s = reinterpret_cast<double*>(smem);
   double* y_s = xp_s + n;
@@ -700,9 +703,14 @@ __device__ __forceinline__ void run_owner(const CtaArgs& a, const CtaLp& L, int 
     }
     // ---- check at iteration it + Lint - 1, then the deferred Halpern step
     const double lam = lambda_at(it + Lint - 1 - restartAt);
-    double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    // pass r: at most one row and one column per virtual thread (R NT <= 1,024)
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < kSumThreads / NT; ++r) {
+      double s[kNumSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+      if (r >= R) {
+        pass_sums<NT>(s, sh, r);
+        continue;
+      }
       const int i = tid + r * NT;
       if (i < m) {
         row_check(s, axpr[r], rl[r], ru[r], a.rfac[L.roff + i], ypr[r], y[r], y0[r]);
@@ -710,18 +718,16 @@ __device__ __forceinline__ void run_owner(const CtaArgs& a, const CtaLp& L, int 
         ax[r] = halpern_step(ax[r], axpr[r], ax0[r], lam, rho);
         y_s[i] = y[r];
       }
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
       const int j = tid + r * NT;
       if (j < n) {
         const double atyp = row_sum(tb[r], te[r], Ti, Tv, yp_s, 0);
         col_check(s, atyp, c[r], lo[r], up[r], a.cfac[L.coff + j], xpr[r], x[r], x0[r]);
         x[r] = halpern_step(x[r], xpr[r], x0[r], lam, rho);
       }
+      pass_sums<NT>(s, sh, r);
     }
     it += Lint - 1;
-    check_decide<NT>(s, sh, a, L, it);
+    check_decide(sh, a, L, it);
     if (sh.ctl.status) break;
     if (sh.ctl.restart) {
       tau = sh.ctl.tau;
@@ -747,7 +753,7 @@ __device__ __forceinline__ void run_owner(const CtaArgs& a, const CtaLp& L, int 
     if (e < n) a.xp[L.coff + e] = xpr[r];
     if (e < m) a.yp[L.roff + e] = ypr[r];
   }
-  write_out<NT>(a, sh.ctl, lp, it);
+  write_out(a, sh.ctl, lp, it);
 }
 
 }  // namespace cta
@@ -760,7 +766,7 @@ __device__ __forceinline__ void run_owner(const CtaArgs& a, const CtaLp& L, int 
 template <int NT, class T = double, int MINB = 1>
 __global__ void __launch_bounds__(NT, MINB) k_lp_cta(CtaArgs a) {
   extern __shared__ __align__(16) unsigned char cta_smem[];
-  __shared__ cta::Shared<NT> sh;
+  __shared__ cta::Shared sh;
   const int lp = a.order[blockIdx.x];
   const CtaLp L = a.lps[lp];
   const int tier = sizeof(T) == sizeof(double) ? L.tier : L.tier32;
@@ -777,7 +783,7 @@ __global__ void __launch_bounds__(NT, MINB) k_lp_cta(CtaArgs a) {
 template <int NT, int R>
 __global__ void __launch_bounds__(NT) k_lp_owner(CtaArgs a) {
   extern __shared__ __align__(16) unsigned char cta_smem[];
-  __shared__ cta::Shared<NT> sh;
+  __shared__ cta::Shared sh;
   const int lp = a.order[blockIdx.x];
   const CtaLp L = a.lps[lp];
   cta::run_owner<NT, R>(a, L, lp, cta_smem, sh);

@@ -382,7 +382,15 @@ struct MultiEngine {
   CtaLp* d_lps = nullptr;
   int32_t* d_order = nullptr;
   CtaOut* d_out = nullptr;
-  int32_t* h_stop = nullptr;  // host-mapped stop flag
+  // Stop flag, read by every block at every check: a device word that the host
+  // sets by a copy on a stream of its own, and only where a deadline or a
+  // cancel flag can set it at all.  (Read from host-mapped memory it cost the
+  // GPU a microsecond per block and check, one after the other over the bus:
+  // 65 ms of the 65 ms of 1,024 small members of 80 checks each.)
+  int32_t* d_stop = nullptr;
+  int32_t* h_one = nullptr;
+  cudaStream_t stop_stream = nullptr;
+  bool may_stop() const { return opt.time_limit > 0 || opt.cancel_flag; }
   // Mixed precision in the CTA form: an FP32 run of every LP (operators and
   // state in FP32), then an FP64 run from each LP's FP32 point.
   bool mixed = false;
@@ -431,7 +439,11 @@ struct MultiEngine {
     PinnedCache::put(h_steps, sizeof(double) * 2 * K);
     PinnedCache::put(h_mask, sizeof(int32_t) * K);
     PinnedCache::put(h_done, sizeof(int32_t) * K);
-    if (h_stop) cudaFreeHost(h_stop);
+    if (stop_stream) {
+      cudaStreamSynchronize(stop_stream);
+      cudaStreamDestroy(stop_stream);
+    }
+    PinnedCache::put(h_one, sizeof(int32_t));
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -937,8 +949,13 @@ struct MultiEngine {
     d_order = upload(order);
     host_order = order;
     d_out = dalloc<CtaOut>(K);
-    B2P_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h_stop), sizeof(int32_t), cudaHostAllocMapped));
-    *h_stop = 0;
+    if (may_stop()) {
+      d_stop = dalloc<int32_t>(1);
+      B2P_CUDA(cudaMemsetAsync(d_stop, 0, sizeof(int32_t), stream));
+      h_one = static_cast<int32_t*>(PinnedCache::get(sizeof(int32_t)));
+      *h_one = 1;
+      B2P_CUDA(cudaStreamCreateWithFlags(&stop_stream, cudaStreamNonBlocking));
+    }
     const int smem = static_cast<int>(cta_smem), osmem = static_cast<int>(cta_owner_smem);
     set_general_attributes<double>(smem);
 #define B2P_OWNER_ATTR(NT, R) \
@@ -1035,7 +1052,7 @@ struct MultiEngine {
     a.entry_check = 0;
     a.stall_checks = 0;
     a.pad = 0;
-    a.stop = h_stop;
+    a.stop = d_stop;
     return a;
   }
 
@@ -1261,16 +1278,15 @@ struct MultiEngine {
 
   // The whole solve is one launch (mixed precision: two, the FP32 run of
   // every LP and the FP64 run from its point); the host only watches the
-  // deadline and the cancel flag and raises the mapped stop flag (read at
-  // every check).
+  // deadline and the cancel flag and raises the stop flag (read at every
+  // check).
   void solve_cta(Clock::time_point deadline_start) {
     const auto t_solve = Clock::now();
     results.assign(K, b2p_result{});
     weights.assign(K, 1.0);
-    *reinterpret_cast<volatile int32_t*>(h_stop) = 0;
     bool raised = false;
     auto wait_for = [&](cudaEvent_t ev) {
-      if (opt.time_limit <= 0 && !opt.cancel_flag) {
+      if (!may_stop()) {
         B2P_CUDA(cudaEventSynchronize(ev));
         return;
       }
@@ -1281,7 +1297,7 @@ struct MultiEngine {
         const bool expired = (opt.cancel_flag && *opt.cancel_flag) ||
                              (opt.time_limit > 0 && seconds_since(deadline_start) >= opt.time_limit);
         if (expired && !raised) {
-          *reinterpret_cast<volatile int32_t*>(h_stop) = 1;
+          B2P_CUDA(cudaMemcpyAsync(d_stop, h_one, sizeof(int32_t), cudaMemcpyHostToDevice, stop_stream));
           raised = true;
         }
         std::this_thread::sleep_for(std::chrono::microseconds(100));
