@@ -1126,7 +1126,7 @@ struct MultiEngine {
     const int64_t probe = std::min<int64_t>(opt.max_iterations, 5 * static_cast<int64_t>(opt.check_every));
     if (probe <= 0 || cands.size() == 1) return;
     const std::vector<int64_t> key{device, K, cta_max_dim, cta_smem32, inst_nnz_total(), opt.check_every,
-                                   opt.cta_threads};
+                                   opt.cta_threads, opt.cta_kernel, opt.cta_smem_limit, opt.cta_layout};
     static std::mutex mu;
     static std::map<std::vector<int64_t>, std::pair<int, int>> chosen;
     {
@@ -1220,7 +1220,8 @@ struct MultiEngine {
   // Variant choice: each candidate runs every LP for five check intervals
   // (tolerance -1: no LP stops early), twice, and the fastest is kept.  The
   // choice is remembered for the process per batch shape (device, LP count,
-  // largest dimension, shared-memory sizes, nonzeros, options), so repeated
+  // largest dimension, shared-memory sizes, nonzeros) and options (the owner
+  // kernel, chosen for a plain batch, cannot run a mixed one's second phase), so repeated
   // batches of one family pay for it once.
   void tune_cta() {
     const auto t0 = Clock::now();
@@ -1235,7 +1236,8 @@ struct MultiEngine {
     int64_t total_nnz = 0;
     for (const CtaLp& c : cta_lps) total_nnz += c.nnz;
     const std::vector<int64_t> key{device, K, cta_max_dim, cta_smem, cta_owner_smem, total_nnz, opt.cta_threads,
-                                   opt.cta_kernel, opt.check_every};
+                                   opt.cta_kernel, opt.check_every, opt.precision, opt.cta_smem_limit,
+                                   opt.cta_layout};
     static std::mutex mu;
     static std::map<std::vector<int64_t>, std::pair<int, int>> chosen;
     {
