@@ -106,6 +106,12 @@ struct CtaArgs {
   const int32_t *sa_base, *sa_idx, *st_base, *st_idx;
   const double *sa_val, *st_val;
   const float *sa_val32, *st_val32;
+  // slab kernel: each operator's rows in order of length (local row numbers,
+  // indexed like the row pointers), and a check's terms per element (five of
+  // every row, five of every column)
+  const int32_t *slab_rows, *slab_cols;
+  double *row_terms, *col_terms;
+  int64_t rows_total, cols_total;
   double tol, rho;
   int64_t max_it;
   int32_t check_every;

@@ -34,6 +34,7 @@
 #include "pdhg_restart.h"
 #include "pdhg_scale.cuh"
 #include "pdhg_cta.cuh"
+#include "pdhg_slab.cuh"
 #include "pdhg_sched.h"
 #include "pdhg_spmv.cuh"
 #include "pdhg_tiled.cuh"
@@ -42,6 +43,13 @@ namespace b2p {
 
 // Instantiated owner-kernel variants: (threads per block, elements per thread).
 #define B2P_OWNER_VARIANTS(X) X(128, 1) X(256, 1) X(512, 1) X(128, 2) X(256, 2) X(512, 2)
+
+// Slab-kernel variants: (threads per block, slices of columns and of rows per
+// warp).
+#define B2P_SLAB_VARIANTS(X) X(512, 2, 1) X(512, 4, 2) X(1024, 2, 1)
+// A variant (threads, r) of the CTA form: r <= 0 general, 1 or 2 owner, else
+// slab with r = slab_code(RC, RR).
+constexpr int slab_code(int rc, int rr) { return 100 + 10 * rc + rr; }
 
 constexpr int kSegRows = 2048;  // rows (or columns) per check-reduction block
 
@@ -404,6 +412,13 @@ struct MultiEngine {
   double *d_x2 = nullptr, *d_y2 = nullptr, *d_ax2 = nullptr;  // the FP64 run's starting point
   CtaLp* d_lps2 = nullptr;
   int32_t* d_order2 = nullptr;
+  // slab kernel: entries of the fullest block, per operator and cluster size 1, 2, 4, 8
+  struct SlabSize {
+    int64_t a[4], t[4];
+  };
+  std::vector<SlabSize> slab_sizes;
+  int32_t *d_slab_rows = nullptr, *d_slab_cols = nullptr;
+  double *d_row_terms = nullptr, *d_col_terms = nullptr;
   std::vector<int32_t> host_order;  // largest LPs first
   static constexpr int kStallChecks = 20;  // FP32 run: checks without a 10% KKT gain before it ends
 
@@ -968,16 +983,121 @@ struct MultiEngine {
       vec_tier = vec_tier || c.tier == kCtaVectors || c.tier == kCtaVectorsPtr;
       if (mixed) vec_tier = vec_tier || c.tier32 == kCtaVectors || c.tier32 == kCtaVectorsPtr;
     }
+    size_slabs(A, AT);
     if (opt.cta_layout != B2P_CTA_LAYOUT_CSR && vec_tier) build_sliced(A, AT);
     if (mixed) setup_cta_fp32();
     tune_cta();
     if (mixed) tune_cta_fp32();
     stats.cta_threads = cta_nt;
-    stats.cta_owned_per_thread = cta_r > 0 ? cta_r : 0;
-    stats.cta_smem_bytes = cta_r > 0 ? cta_owner_smem : cta_smem;
+    stats.cta_owned_per_thread = cta_r >= 100 ? (cta_r - 100) / 10 : cta_r > 0 ? cta_r : 0;
+    stats.cta_smem_bytes = cta_r >= 100 ? slab_fit(cta_nt, cta_r, 8).smem : cta_r > 0 ? cta_owner_smem : cta_smem;
     stats.cta_lps_smem = n_all;
     stats.cta_lps_vectors = n_vec;
     stats.cta_sliced = d_sa_base != nullptr && cta_r <= 0;
+  }
+
+  // ---- slab kernel (pdhg_slab.cuh) ----
+
+  void size_slabs(const HostCsr& A, const HostCsr& AT) {
+    slab_sizes.assign(ops, SlabSize{});
+    std::vector<int32_t> rows(Mo), cols(No);
+    for (int b = 0; b < ops; ++b) {
+      const int32_t *ap = A.ptr.data() + roff[b], *tp = AT.ptr.data() + coff[b];
+      int32_t *ro = rows.data() + roff[b], *co = cols.data() + coff[b];
+      slab_order(ap, P[b].m, ro);
+      slab_order(tp, P[b].n, co);
+      for (int q = 0; q < 4; ++q) {
+        slab_sizes[b].a[q] = slab_entries(ap, P[b].m, ro, 1 << q);
+        slab_sizes[b].t[q] = slab_entries(tp, P[b].n, co, 1 << q);
+      }
+    }
+    d_slab_rows = upload(rows);
+    d_slab_cols = upload(cols);
+    d_row_terms = dalloc<double>(static_cast<size_t>(M) * kRowSums);
+    d_col_terms = dalloc<double>(static_cast<size_t>(N) * kRowSums);
+  }
+
+  // The smallest cluster on which every LP fits a variant (blocks 0: none).
+  struct SlabFit {
+    int blocks = 0;
+    int64_t smem = 0;
+  };
+  SlabFit slab_fit(int nt, int r, int esize) const {
+    const int rc = (r - 100) / 10, rr = (r - 100) % 10, warps = nt / 32;
+    const int64_t budget = cta_budget();
+    for (int q = 0; q < 4; ++q) {
+      const int C = 1 << q;
+      int64_t need = 0;
+      bool ok = true;
+      for (int b = 0; b < K && ok; ++b) {
+        const int64_t m = P[b].m, n = P[b].n;
+        const SlabSize& z = slab_sizes[b < ops ? b : 0];
+        ok = m < 65536 && n < 65536 && (n + 32 * C - 1) / (32 * C) <= rc * warps &&
+             (m + 32 * C - 1) / (32 * C) <= rr * warps;
+        need = std::max(need, slab_smem_bytes(m, n, z.a[q], z.t[q], esize));
+      }
+      if (ok && need <= budget) return SlabFit{C, need};
+    }
+    return SlabFit{};
+  }
+
+  // Launches a slab variant on its cluster size; false if there is no such
+  // variant.  `probe`: only whether it can run.
+  template <class T>
+  bool launch_slab(int nt, int r, const CtaArgs& a, unsigned lps, bool probe = false) {
+    const SlabFit fit = slab_fit(nt, r, sizeof(T));
+    if (fit.blocks == 0) return false;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(lps * fit.blocks);
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = static_cast<size_t>(fit.smem);
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = fit.blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    bool found = false;
+#define B2P_SLAB_LAUNCH(NT, RC, RR)                                                                              \
+  if (!found && nt == NT && r == slab_code(RC, RR)) {                                                            \
+    const auto fn = k_lp_slab<NT, RC, RR, T>;                                                                    \
+    B2P_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cta_budget()))); \
+    if (probe) {                                                                                                 \
+      int clusters = 0;                                                                                          \
+      found = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;               \
+      if (!found) cudaGetLastError();                                                                            \
+    } else {                                                                                                     \
+      B2P_CUDA(cudaLaunchKernelEx(&cfg, fn, a, fit.blocks));                                                     \
+      found = true;                                                                                              \
+    }                                                                                                            \
+  }
+    B2P_SLAB_VARIANTS(B2P_SLAB_LAUNCH)
+#undef B2P_SLAB_LAUNCH
+    return found;
+  }
+
+  // Slab variants that can run this batch, where the options leave the choice:
+  // for LPs whose operators do not fit one block (those that do fill the SMs
+  // better one block each: 1,024 members of 164 x 324 2.2 ms in either form,
+  // 148 0.41 / 0.45), and only while every LP's cluster runs at once (30
+  // members of 1,692 x 3,528, 320 iterations, general / slab: 3.2 / 1.2 ms; 296
+  // of them 6.4 / 7.3: the SMs are busy either way).
+  template <class T>
+  void slab_candidates(std::vector<std::pair<int, int>>& c) {
+    if (opt.cta_kernel != B2P_CTA_AUTO || opt.cta_smem_limit > 0 || opt.cta_layout == B2P_CTA_LAYOUT_CSR) return;
+    bool large = false;
+    for (const CtaLp& l : cta_lps) large = large || (sizeof(T) == 8 ? l.tier : l.tier32) != kCtaAll;
+    int sms = 0;
+    B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (!large) return;
+#define B2P_SLAB_CAND(NT, RC, RR)                                                                                  \
+  if ((opt.cta_threads == 0 || opt.cta_threads == NT) &&                                                           \
+      static_cast<int64_t>(K) * slab_fit(NT, slab_code(RC, RR), sizeof(T)).blocks <= sms &&                        \
+      launch_slab<T>(NT, slab_code(RC, RR), CtaArgs{}, static_cast<unsigned>(K), true))                            \
+    c.emplace_back(NT, slab_code(RC, RR));
+    B2P_SLAB_VARIANTS(B2P_SLAB_CAND)
+#undef B2P_SLAB_CAND
   }
 
   // Sliced-ELL copies of A and A^T for the CTA form: per LP (LP 0 alone when
@@ -1045,6 +1165,9 @@ struct MultiEngine {
     a.x32 = v32[0], a.xp32 = v32[1], a.x032 = v32[2];
     a.y32 = v32[3], a.yp32 = v32[4], a.y032 = v32[5];
     a.ax32 = v32[6], a.axp32 = v32[7], a.ax032 = v32[8];
+    a.slab_rows = d_slab_rows, a.slab_cols = d_slab_cols;
+    a.row_terms = d_row_terms, a.col_terms = d_col_terms;
+    a.rows_total = M, a.cols_total = N;
     a.tol = tol;
     a.rho = opt.reflection;
     a.max_it = max_it;
@@ -1113,6 +1236,10 @@ struct MultiEngine {
     B2P_CUDA(cudaGetLastError());
   }
   void launch_cta32(int nt, int r, const CtaArgs& a, unsigned grid) {
+    if (r >= 100) {
+      if (!launch_slab<float>(nt, r, a, grid)) throw Error(B2P_ERR_INVALID, "no such CTA kernel variant");
+      return;
+    }
     launch_general<float>(nt, r, a, grid, static_cast<size_t>(cta_smem32));
   }
 
@@ -1120,7 +1247,8 @@ struct MultiEngine {
   // check intervals, twice; the fastest is kept (remembered per batch shape).
   void tune_cta_fp32() {
     const auto t0 = Clock::now();
-    const std::vector<std::pair<int, int>> cands = general_candidates();
+    std::vector<std::pair<int, int>> cands = general_candidates();
+    slab_candidates<float>(cands);
     cta_nt32 = cands.front().first;
     cta_r32 = cands.front().second;
     const int64_t probe = std::min<int64_t>(opt.max_iterations, 5 * static_cast<int64_t>(opt.check_every));
@@ -1171,6 +1299,8 @@ struct MultiEngine {
     const unsigned grid = static_cast<unsigned>(lps < 0 ? K : lps);
     if (r <= 0) {
       launch_general<double>(nt, r, a, grid, static_cast<size_t>(cta_smem));
+    } else if (r >= 100) {
+      if (!launch_slab<double>(nt, r, a, grid)) throw Error(B2P_ERR_INVALID, "no such CTA kernel variant");
     } else {
       const size_t smem = static_cast<size_t>(cta_owner_smem);
       bool launched = false;
@@ -1200,7 +1330,7 @@ struct MultiEngine {
   // 512 and 1,024 threads (256 and 512 also compiled for 1,024 threads per
   // SM), and the owner kernel where every LP's rows and columns fit R per
   // thread and its data fits in shared memory.
-  std::vector<std::pair<int, int>> cta_candidates() const {
+  std::vector<std::pair<int, int>> cta_candidates() {
     const int want = opt.cta_kernel;  // B2P_CTA_*
     if (want < B2P_CTA_AUTO || want > B2P_CTA_OWNER2) throw Error(B2P_ERR_INVALID, "unknown cta_kernel");
     std::vector<std::pair<int, int>> c;
@@ -1213,6 +1343,7 @@ struct MultiEngine {
       B2P_OWNER_VARIANTS(B2P_OWNER_CAND)
 #undef B2P_OWNER_CAND
     }
+    slab_candidates<double>(c);
     if (c.empty()) throw Error(B2P_ERR_INVALID, "no CTA kernel variant fits these LPs and options");
     return c;
   }
