@@ -11,6 +11,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <optional>
 #include <random>
 #include <vector>
 
@@ -352,7 +353,7 @@ struct Mlp {
   __nv_bfloat16* gb[2] = {nullptr, nullptr};
   double* partial = nullptr;                  // kLossBlocks
   double* d_loss = nullptr;                   // [0] last loss, [1..] epoch sums
-  ErrorWord error;
+  std::optional<ErrorWord> error;             // once there is a device
   std::vector<void*> owned;
 
   ~Mlp() {
@@ -410,6 +411,7 @@ struct Mlp {
       gb[i] = alloc<__nv_bfloat16>(static_cast<size_t>(mb) * wmax);
     }
     partial = alloc<double>(kLossBlocks);
+    error.emplace();
     set_gemm_attributes();
     reset_moments();
     B2P_CUDA(cudaStreamSynchronize(stream));
@@ -424,7 +426,7 @@ struct Mlp {
   GemmArgs gemm_base() const {
     GemmArgs g{};
     g.alpha = 1.0f;
-    g.error = error.device();
+    g.error = error->device();
     return g;
   }
 
@@ -505,7 +507,7 @@ struct Mlp {
     }
   }
 
-  void check_error() { error.check(stream); }
+  void check_error() { error->check(stream); }
 
   void set_params(const float* hp) {
     B2P_CUDA(cudaSetDevice(device));

@@ -105,3 +105,11 @@ def test_host_side_argument_checks():
         pdhg.certifyLp(lp, np.zeros(lp.num_cols), np.zeros(lp.num_rows - 1))
     with pytest.raises(ValueError):
         pdhg.kktResidual(lp, np.zeros(lp.num_cols + 2), np.zeros(lp.num_rows))
+
+
+@pytest.mark.skipif(_gpu_present(), reason="checks the no-device path")
+def test_network_without_device(engine_lib):
+    from pramana_b200.mlp import MlpNetwork
+    with pytest.raises(_lib.B2pError) as e:
+        MlpNetwork((16, 512, 128), max_batch=512, seed=0)
+    assert e.value.code == 3
