@@ -43,6 +43,19 @@ __device__ __forceinline__ double member_beta(const MemberData& d, const double*
   return d.rescale ? __dadd_rn(1.0, __dsqrt_rn(sums[MS_SB])) : 1.0;
 }
 
+// Blocks of a member along the grid's y dimension, which holds 65,535: enough
+// for one thread per element of a member of 16.7 M, whose threads take several
+// beyond that.
+constexpr int64_t kMemberMaxBlocks = 65535;
+inline unsigned member_grid_y(int64_t elements) {
+  const int64_t blocks = (elements + kBlock - 1) / kBlock;
+  return static_cast<unsigned>(blocks < 1 ? 1 : blocks < kMemberMaxBlocks ? blocks : kMemberMaxBlocks);
+}
+__device__ __forceinline__ int64_t member_first() {
+  return static_cast<int64_t>(blockIdx.y) * kBlock + threadIdx.x;
+}
+__device__ __forceinline__ int64_t member_stride() { return static_cast<int64_t>(gridDim.y) * kBlock; }
+
 __device__ __forceinline__ double add_in_order(double t, const double* term, int count) {
 #pragma unroll 16
   for (int i = 0; i < count; ++i) t = __dadd_rn(t, term[i]);
@@ -100,22 +113,22 @@ __global__ void __launch_bounds__(kBlock) k_member_columns(MemberData d, const d
                                                            double* __restrict__ cfac) {
   const int b = blockIdx.x;
   const int32_t c0 = d.coff[b], n = d.coff[b + 1] - c0;
-  const int64_t j = static_cast<int64_t>(blockIdx.y) * kBlock + threadIdx.x;
-  if (j >= n) return;
   const double* sb = sums + static_cast<int64_t>(b) * kMemberSums;
   const double gamma = member_gamma(d, sb), beta = member_beta(d, sb);
-  const double s = d.Cs[(d.shared ? 0 : c0) + j];
-  const int64_t t = c0 + j;
-  const double l = d.lower[t], u = d.upper[t];
-  cfac[t] = __ddiv_rn(gamma, s);
-  c[t] = __ddiv_rn(__dmul_rn(d.cost[t], s), gamma);
-  const double lv = member_finite(l) ? __ddiv_rn(__ddiv_rn(l, s), beta) : -INFINITY;
-  const double uv = member_finite(u) ? __ddiv_rn(__ddiv_rn(u, s), beta) : INFINITY;
-  lo[t] = lv;
-  up[t] = uv;
-  double v = (0.0 < lv) ? lv : 0.0;
-  v = (uv < v) ? uv : v;
-  x[t] = v;
+  for (int64_t j = member_first(); j < n; j += member_stride()) {
+    const double s = d.Cs[(d.shared ? 0 : c0) + j];
+    const int64_t t = c0 + j;
+    const double l = d.lower[t], u = d.upper[t];
+    cfac[t] = __ddiv_rn(gamma, s);
+    c[t] = __ddiv_rn(__dmul_rn(d.cost[t], s), gamma);
+    const double lv = member_finite(l) ? __ddiv_rn(__ddiv_rn(l, s), beta) : -INFINITY;
+    const double uv = member_finite(u) ? __ddiv_rn(__ddiv_rn(u, s), beta) : INFINITY;
+    lo[t] = lv;
+    up[t] = uv;
+    double v = (0.0 < lv) ? lv : 0.0;
+    v = (uv < v) ? uv : v;
+    x[t] = v;
+  }
 }
 
 // grid = (members, blocks of rows): scaled sides, the check's row factors.
@@ -124,15 +137,15 @@ __global__ void __launch_bounds__(kBlock) k_member_rows(MemberData d, const doub
                                                         double* __restrict__ rfac) {
   const int b = blockIdx.x;
   const int32_t r0 = d.roff[b], m = d.roff[b + 1] - r0;
-  const int64_t i = static_cast<int64_t>(blockIdx.y) * kBlock + threadIdx.x;
-  if (i >= m) return;
   const double beta = member_beta(d, sums + static_cast<int64_t>(b) * kMemberSums);
-  const double s = d.R[(d.shared ? 0 : r0) + i];
-  const int64_t t = r0 + i;
-  const double l = d.rl[t], u = d.ru[t];
-  rfac[t] = __ddiv_rn(beta, s);
-  rl[t] = member_finite(l) ? __ddiv_rn(__dmul_rn(l, s), beta) : -INFINITY;
-  ru[t] = member_finite(u) ? __ddiv_rn(__dmul_rn(u, s), beta) : INFINITY;
+  for (int64_t i = member_first(); i < m; i += member_stride()) {
+    const double s = d.R[(d.shared ? 0 : r0) + i];
+    const int64_t t = r0 + i;
+    const double l = d.rl[t], u = d.ru[t];
+    rfac[t] = __ddiv_rn(beta, s);
+    rl[t] = member_finite(l) ? __ddiv_rn(__dmul_rn(l, s), beta) : -INFINITY;
+    ru[t] = member_finite(u) ? __ddiv_rn(__dmul_rn(u, s), beta) : INFINITY;
+  }
 }
 
 // grid = (members, 2): the norms of the scaled LP.
@@ -168,10 +181,12 @@ __global__ void __launch_bounds__(kBlock) k_member_answers(MemberData d, int32_t
                                                            double* __restrict__ y) {
   const int b = first + blockIdx.x;
   const int32_t c0 = d.coff[b], n = d.coff[b + 1] - c0, r0 = d.roff[b], m = d.roff[b + 1] - r0;
-  const int64_t i = static_cast<int64_t>(blockIdx.y) * kBlock + threadIdx.x;
   const double* sb = sums + static_cast<int64_t>(b) * kMemberSums;
-  if (i < n) x[c0 + i] = __dmul_rn(__dmul_rn(xp[c0 + i], d.Cs[(d.shared ? 0 : c0) + i]), member_beta(d, sb));
-  if (i < m) y[r0 + i] = __dmul_rn(__dmul_rn(yp[r0 + i], d.R[(d.shared ? 0 : r0) + i]), member_gamma(d, sb));
+  const double gamma = member_gamma(d, sb), beta = member_beta(d, sb);
+  for (int64_t i = member_first(); i < (n > m ? n : m); i += member_stride()) {
+    if (i < n) x[c0 + i] = __dmul_rn(__dmul_rn(xp[c0 + i], d.Cs[(d.shared ? 0 : c0) + i]), beta);
+    if (i < m) y[r0 + i] = __dmul_rn(__dmul_rn(yp[r0 + i], d.R[(d.shared ? 0 : r0) + i]), gamma);
+  }
 }
 
 }  // namespace b2p

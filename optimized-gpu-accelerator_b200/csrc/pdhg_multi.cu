@@ -649,11 +649,11 @@ struct MultiEngine {
     B2P_CUDA(cudaGetLastError());
   }
 
-  // Blocks along y for one thread per column and row of the largest LP.
+  // Blocks along y for the columns and rows of the largest LP.
   unsigned member_blocks(bool cols, bool rows) const {
     int32_t most = 1;
     for (int b = 0; b < K; ++b) most = std::max(most, std::max(cols ? P[b].n : 0, rows ? P[b].m : 0));
-    return (most + kBlock - 1) / kBlock;
+    return member_grid_y(most);
   }
 
   // The caller's costs, bounds and sides to the device (through a page-locked

@@ -70,3 +70,20 @@ def test_degenerate_members(form):
     r = pdhg.solvePdhgMulti([empty, empty, lp], po)
     assert np.array_equal(r[0].x, r[1].x) and abs(r[0].objective + 1.0) <= 1e-6
     assert np.max(np.abs(r[2].x - alone.x)) <= 1e-9 * max(1.0, np.max(np.abs(alone.x)))
+
+
+def test_more_elements_than_the_grid_has_threads():
+    """One LP of 65,535 blocks of 256 columns and 300 more, few of them in its three rows."""
+    m, n, used = 3, 65535 * 256 + 300, 8
+    rng = np.random.default_rng(26)
+    at = np.r_[0:used // 2, n - used // 2:n]  # both ends
+    counts = np.zeros(n, dtype=np.int64)
+    counts[at] = 1
+    lp = Model(num_rows=m, num_cols=n, start=np.concatenate([[0], np.cumsum(counts)]), index=np.arange(used) % m,
+               value=rng.uniform(1.0, 2.0, size=used), col_cost=rng.standard_normal(n), col_lower=np.zeros(n),
+               col_upper=np.ones(n), row_lower=np.full(m, 0.5), row_upper=np.full(m, np.inf))
+    po = pdhg.PdhgOptions(tolerance=1e-30, maxIterations=3, multiForm=_lib.MULTI_GRID)
+    got = pdhg.solvePdhgMulti([lp], po)[0]
+    want = O.solve(lp, "oracle", tolerance=1e-30, max_iterations=3)
+    # three steps of separately rounded arithmetic over sums of at most three terms
+    assert np.max(np.abs(got.x - want.x)) <= 1e-12 and np.max(np.abs(got.rowDual - want.y)) <= 1e-12
