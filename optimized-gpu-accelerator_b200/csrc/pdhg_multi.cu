@@ -983,7 +983,7 @@ struct MultiEngine {
       vec_tier = vec_tier || c.tier == kCtaVectors || c.tier == kCtaVectorsPtr;
       if (mixed) vec_tier = vec_tier || c.tier32 == kCtaVectors || c.tier32 == kCtaVectorsPtr;
     }
-    size_slabs(A, AT);
+    if (slab_wanted()) size_slabs(A, AT);
     if (opt.cta_layout != B2P_CTA_LAYOUT_CSR && vec_tier) build_sliced(A, AT);
     if (mixed) setup_cta_fp32();
     tune_cta();
@@ -998,6 +998,22 @@ struct MultiEngine {
 
   // ---- slab kernel (pdhg_slab.cuh) ----
 
+  int sm_count() const {
+    int sms = 0;
+    B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    return sms;
+  }
+  // Whether the options leave the choice and the batch is one that
+  // slab_candidates can take.
+  bool slab_wanted() const {
+    if (opt.cta_kernel != B2P_CTA_AUTO || opt.cta_smem_limit > 0 || opt.cta_layout == B2P_CTA_LAYOUT_CSR) return false;
+    bool large = false;
+    for (const CtaLp& l : cta_lps) large = large || l.tier != kCtaAll || (mixed && l.tier32 != kCtaAll);
+    return large && K <= sm_count();
+  }
+
+  // The order of the rows, the entries each cluster size needs, and, where
+  // some variant takes the batch, the checks' scratch.
   void size_slabs(const HostCsr& A, const HostCsr& AT) {
     slab_sizes.assign(ops, SlabSize{});
     std::vector<int32_t> rows(Mo), cols(No);
@@ -1011,10 +1027,21 @@ struct MultiEngine {
         slab_sizes[b].t[q] = slab_entries(tp, P[b].n, co, 1 << q);
       }
     }
-    d_slab_rows = upload(rows);
-    d_slab_cols = upload(cols);
-    d_row_terms = dalloc<double>(static_cast<size_t>(M) * kRowSums);
-    d_col_terms = dalloc<double>(static_cast<size_t>(N) * kRowSums);
+    const int64_t sms = sm_count();
+    bool any = false;
+#define B2P_SLAB_ANY(NT, RC, RR)                                                        \
+  for (const int esize : {8, 4}) {                                                      \
+    const int64_t blocks = slab_fit(NT, slab_code(RC, RR), esize).blocks;               \
+    any = any || (blocks > 0 && K * blocks <= sms);                                     \
+  }
+    B2P_SLAB_VARIANTS(B2P_SLAB_ANY)
+#undef B2P_SLAB_ANY
+    if (any) {
+      d_slab_rows = upload(rows);
+      d_slab_cols = upload(cols);
+      d_row_terms = dalloc<double>(static_cast<size_t>(M) * kRowSums);
+      d_col_terms = dalloc<double>(static_cast<size_t>(N) * kRowSums);
+    }
   }
 
   // The smallest cluster on which every LP fits a variant (blocks 0: none).
@@ -1085,11 +1112,10 @@ struct MultiEngine {
   // of them 6.4 / 7.3: the SMs are busy either way).
   template <class T>
   void slab_candidates(std::vector<std::pair<int, int>>& c) {
-    if (opt.cta_kernel != B2P_CTA_AUTO || opt.cta_smem_limit > 0 || opt.cta_layout == B2P_CTA_LAYOUT_CSR) return;
+    if (!d_slab_cols) return;
     bool large = false;
     for (const CtaLp& l : cta_lps) large = large || (sizeof(T) == 8 ? l.tier : l.tier32) != kCtaAll;
-    int sms = 0;
-    B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int sms = sm_count();
     if (!large) return;
 #define B2P_SLAB_CAND(NT, RC, RR)                                                                                  \
   if ((opt.cta_threads == 0 || opt.cta_threads == NT) &&                                                           \
@@ -1243,6 +1269,12 @@ struct MultiEngine {
     launch_general<float>(nt, r, a, grid, static_cast<size_t>(cta_smem32));
   }
 
+  // Whether a remembered choice can run this batch: which slab variants can
+  // depends on how long each row is, which the shape does not tell.
+  static bool is_candidate(const std::vector<std::pair<int, int>>& cands, const std::pair<int, int>& v) {
+    return std::find(cands.begin(), cands.end(), v) != cands.end();
+  }
+
   // Threads per block of the FP32 run: each count runs every LP for five
   // check intervals, twice; the fastest is kept (remembered per batch shape).
   void tune_cta_fp32() {
@@ -1260,7 +1292,7 @@ struct MultiEngine {
     {
       std::lock_guard<std::mutex> lock(mu);
       const auto it = chosen.find(key);
-      if (it != chosen.end()) {
+      if (it != chosen.end() && is_candidate(cands, it->second)) {
         cta_nt32 = it->second.first;
         cta_r32 = it->second.second;
         return;
@@ -1374,7 +1406,7 @@ struct MultiEngine {
     {
       std::lock_guard<std::mutex> lock(mu);
       const auto it = chosen.find(key);
-      if (it != chosen.end()) {
+      if (it != chosen.end() && is_candidate(cands, it->second)) {
         cta_nt = it->second.first;
         cta_r = it->second.second;
         return;

@@ -49,3 +49,22 @@ def test_deadline():
     res = pdhg.solvePdhgMulti(lps, pdhg.PdhgOptions(tolerance=1e-30, maxIterations=200_000_000, timeLimit=0.5,
                                                     multiForm=_lib.MULTI_CTA))
     assert {r.status for r in res} == {"TimeLimit"}
+
+
+def test_choice_of_another_batch_of_the_same_shape():
+    """A batch with the sizes of an earlier one that the slab kernel cannot hold: one row of 2,500 entries, whose slice
+    of 32 rows would be 800 KB."""
+    m, n, per = 1500, 2500, 6
+    rng = np.random.default_rng(56)
+
+    def lp(long_row):
+        rows = np.sort(rng.permuted(np.tile(np.arange(1, m), (n, 1)), axis=1)[:, :per], axis=1)
+        if long_row:
+            rows[:, 0] = 0
+        base = G.random_lp(m, n, 3.0, m // 2, 57)
+        return type(base)(num_rows=m, num_cols=n, start=np.arange(n + 1) * per, index=rows.ravel(),
+                          value=rng.standard_normal(n * per), col_cost=base.col_cost, col_lower=base.col_lower,
+                          col_upper=base.col_upper, row_lower=base.row_lower, row_upper=base.row_upper)
+
+    for long_row in (False, True, False):
+        _check([lp(long_row) for _ in range(3)], 0, 130)
