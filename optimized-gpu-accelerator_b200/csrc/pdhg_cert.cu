@@ -17,7 +17,8 @@
 //    operation is rounded in the safe direction by the hardware's directed-
 //    rounding instructions (__dadd_rd, __dmul_ru, __ddiv_rd, ...), so the
 //    bounds contain every feasible point of the exact LP and need no safety
-//    margin.  Rounds repeat until no bound of a case moves by more than
+//    margin.  LPs that fit a block's shared memory run all their rounds in one
+//    launch, one block a case (k_ib_block).  Rounds repeat until no bound of a case moves by more than
 //    kIbStep relative (or kIbMaxRounds); a case whose bounds cross is
 //    infeasible and keeps the bounds it had.
 // 2. The primal half of the verdict (b2p_certify_lp).  Per (row, case) the
@@ -148,64 +149,48 @@ __device__ __forceinline__ void block_combine(double& q, int32_t& at, TwoWord& s
 
 // ---- implied bounds --------------------------------------------------------
 
-// Per (row i, case b): smallest / largest activity over the finite
-// contributions, rounded down / up, and how many contributions are infinite.
-__global__ void __launch_bounds__(kBlock) k_ib_activity(int32_t m, int32_t n, CsrView A, const double* __restrict__ lo,
-                                                        const double* __restrict__ up, const int32_t* __restrict__ live,
-                                                        const int32_t* __restrict__ infeasible,
-                                                        double* __restrict__ act_lo, double* __restrict__ act_hi,
-                                                        int32_t* __restrict__ inf_lo, int32_t* __restrict__ inf_hi) {
-  const int b = blockIdx.y;
-  if (!live[b] || infeasible[b]) return;
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const double* lb = lo + static_cast<int64_t>(b) * n;
-  const double* ub = up + static_cast<int64_t>(b) * n;
-  double s_lo = 0.0, s_hi = 0.0;
-  int32_t c_lo = 0, c_hi = 0;
-  for (int p = A.ptr[i]; p < A.ptr[i + 1]; ++p) {
-    const double a = A.val[p];
+// A row's smallest / largest activity over the finite contributions, rounded
+// down / up, and how many contributions are infinite.
+struct RowActivity {
+  double lo, hi;
+  int32_t inf_lo, inf_hi;
+};
+__device__ __forceinline__ RowActivity ib_activity(int beg, int end, const int32_t* __restrict__ idx,
+                                                   const double* __restrict__ val, const double* __restrict__ lb,
+                                                   const double* __restrict__ ub) {
+  RowActivity s{0.0, 0.0, 0, 0};
+  for (int p = beg; p < end; ++p) {
+    const double a = val[p];
     if (a == 0.0) continue;
-    const int32_t j = A.idx[p];
+    const int32_t j = idx[p];
     const double at_min = a > 0.0 ? lb[j] : ub[j];  // the bound where a*x_j is smallest
     const double at_max = a > 0.0 ? ub[j] : lb[j];
     if (cert::fin(at_min))
-      s_lo = __dadd_rd(s_lo, __dmul_rd(a, at_min));
+      s.lo = __dadd_rd(s.lo, __dmul_rd(a, at_min));
     else
-      ++c_lo;
+      ++s.inf_lo;
     if (cert::fin(at_max))
-      s_hi = __dadd_ru(s_hi, __dmul_ru(a, at_max));
+      s.hi = __dadd_ru(s.hi, __dmul_ru(a, at_max));
     else
-      ++c_hi;
+      ++s.inf_hi;
   }
-  const int64_t t = static_cast<int64_t>(b) * m + i;
-  act_lo[t] = s_lo;
-  act_hi[t] = s_hi;
-  inf_lo[t] = c_lo;
-  inf_hi[t] = c_hi;
+  return s;
 }
 
-// Per (column j, case b): the bounds each row of the column implies, taken
-// together with the column's own; AT is the CSR of A^T (the column's rows).
-__global__ void __launch_bounds__(kBlock) k_ib_tighten(int32_t n, int32_t m, CsrView AT, const double* __restrict__ rl,
-                                                       const double* __restrict__ ru,
-                                                       const double* __restrict__ act_lo,
-                                                       const double* __restrict__ act_hi,
-                                                       const int32_t* __restrict__ inf_lo,
-                                                       const int32_t* __restrict__ inf_hi, double* __restrict__ lo,
-                                                       double* __restrict__ up, const int32_t* __restrict__ live,
-                                                       int32_t* __restrict__ progress, int32_t* __restrict__ infeasible) {
-  const int b = blockIdx.y;
-  if (!live[b] || infeasible[b]) return;
-  const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const int64_t t = static_cast<int64_t>(b) * n + j;
-  const double l = lo[t], u = up[t];
+enum IbMove : int { kIbStays = 0, kIbMoves = 1, kIbCrosses = 2 };
+
+// The bounds [l, u] of a column taken together with what each of its rows
+// implies (beg .. end of AT, the CSR of A^T; row vectors of the column's case).
+__device__ __forceinline__ IbMove ib_tighten(int beg, int end, const int32_t* __restrict__ idx,
+                                             const double* __restrict__ val, const double* __restrict__ rl,
+                                             const double* __restrict__ ru, const double* __restrict__ act_lo,
+                                             const double* __restrict__ act_hi, const int32_t* __restrict__ inf_lo,
+                                             const int32_t* __restrict__ inf_hi, double& l, double& u) {
   double nl = l, nu = u;
-  for (int p = AT.ptr[j]; p < AT.ptr[j + 1]; ++p) {
-    const double a = AT.val[p];
+  for (int p = beg; p < end; ++p) {
+    const double a = val[p];
     if (a == 0.0) continue;
-    const int64_t r = static_cast<int64_t>(b) * m + AT.idx[p];
+    const int32_t r = idx[p];
     const double L = rl[r], U = ru[r];
     const double at_min = a > 0.0 ? l : u, at_max = a > 0.0 ? u : l;
     // the other entries' smallest activity (a lower bound of it) ...
@@ -251,40 +236,163 @@ __global__ void __launch_bounds__(kBlock) k_ib_tighten(int32_t n, int32_t m, Csr
       }
     }
   }
-  if (cert::fin(nl) && cert::fin(nu) && nl > nu) {
+  if (cert::fin(nl) && cert::fin(nu) && nl > nu) return kIbCrosses;
+  const bool moved_lo = cert::fin(nl) && (!cert::fin(l) || nl - l > kIbStep * (1.0 + fabs(nl)));
+  const bool moved_up = cert::fin(nu) && (!cert::fin(u) || u - nu > kIbStep * (1.0 + fabs(nu)));
+  if (cert::fin(nl) && (!cert::fin(l) || nl > l)) l = nl;
+  if (cert::fin(nu) && (!cert::fin(u) || nu < u)) u = nu;
+  return moved_lo || moved_up ? kIbMoves : kIbStays;
+}
+
+// The activities of every (row, case).
+__global__ void __launch_bounds__(kBlock) k_ib_activity(int32_t m, int32_t n, CsrView A, const double* __restrict__ lo,
+                                                        const double* __restrict__ up, const int32_t* __restrict__ live,
+                                                        const int32_t* __restrict__ infeasible,
+                                                        double* __restrict__ act_lo, double* __restrict__ act_hi,
+                                                        int32_t* __restrict__ inf_lo, int32_t* __restrict__ inf_hi) {
+  const int b = blockIdx.y;
+  if (!live[b] || infeasible[b]) return;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const int64_t c = static_cast<int64_t>(b) * n, t = static_cast<int64_t>(b) * m + i;
+  const RowActivity s = ib_activity(A.ptr[i], A.ptr[i + 1], A.idx, A.val, lo + c, up + c);
+  act_lo[t] = s.lo;
+  act_hi[t] = s.hi;
+  inf_lo[t] = s.inf_lo;
+  inf_hi[t] = s.inf_hi;
+}
+
+// The bounds of every (column, case).
+__global__ void __launch_bounds__(kBlock) k_ib_tighten(int32_t n, int32_t m, CsrView AT, const double* __restrict__ rl,
+                                                       const double* __restrict__ ru,
+                                                       const double* __restrict__ act_lo,
+                                                       const double* __restrict__ act_hi,
+                                                       const int32_t* __restrict__ inf_lo,
+                                                       const int32_t* __restrict__ inf_hi, double* __restrict__ lo,
+                                                       double* __restrict__ up, const int32_t* __restrict__ live,
+                                                       int32_t* __restrict__ progress, int32_t* __restrict__ infeasible) {
+  const int b = blockIdx.y;
+  if (!live[b] || infeasible[b]) return;
+  const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int64_t t = static_cast<int64_t>(b) * n + j, r = static_cast<int64_t>(b) * m;
+  const double l0 = lo[t], u0 = up[t];
+  double l = l0, u = u0;
+  const IbMove move = ib_tighten(AT.ptr[j], AT.ptr[j + 1], AT.idx, AT.val, rl + r, ru + r, act_lo + r, act_hi + r,
+                                 inf_lo + r, inf_hi + r, l, u);
+  if (move == kIbCrosses) {
     infeasible[b] = 1;  // no point of the exact LP satisfies the rows: the case is infeasible
     return;
   }
-  const bool moved_lo = cert::fin(nl) && (!cert::fin(l) || nl - l > kIbStep * (1.0 + fabs(nl)));
-  const bool moved_up = cert::fin(nu) && (!cert::fin(u) || u - nu > kIbStep * (1.0 + fabs(nu)));
-  if (cert::fin(nl) && (!cert::fin(l) || nl > l)) lo[t] = nl;
-  if (cert::fin(nu) && (!cert::fin(u) || nu < u)) up[t] = nu;
-  if (moved_lo || moved_up) progress[b] = 1;
+  if (l != l0) lo[t] = l;
+  if (u != u0) up[t] = u;
+  if (move == kIbMoves) progress[b] = 1;
 }
+
+// All rounds of a case in one block, grid = k: operators, bounds, sides and
+// activities in shared memory.  Rounds number in the hundreds, and two
+// launches and their gaps (5.5 us) are all that a round of the grid form is on
+// a small LP; here it is two block barriers and the longest row's and column's
+// serial chains.  The same expressions in the same order: the same bounds.
+__global__ void __launch_bounds__(1024) k_ib_block(int32_t m, int32_t n, int32_t nnz, CsrView A, CsrView AT,
+                                                   const double* __restrict__ rl, const double* __restrict__ ru,
+                                                   double* __restrict__ lo, double* __restrict__ up) {
+  extern __shared__ __align__(16) unsigned char ib_smem[];
+  double* sl = reinterpret_cast<double*>(ib_smem);
+  double *su = sl + n, *srl = su + n, *sru = srl + m, *alo = sru + m, *ahi = alo + m, *av = ahi + m, *tv = av + nnz;
+  int32_t* ilo = reinterpret_cast<int32_t*>(tv + nnz);
+  int32_t *ihi = ilo + m, *ai = ihi + m, *ti = ai + nnz, *ap = ti + nnz, *tp = ap + m + 1;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int64_t c = static_cast<int64_t>(blockIdx.x) * n, r = static_cast<int64_t>(blockIdx.x) * m;
+  for (int j = tid; j < n; j += nt) {
+    sl[j] = lo[c + j];
+    su[j] = up[c + j];
+  }
+  for (int i = tid; i < m; i += nt) {
+    srl[i] = rl[r + i];
+    sru[i] = ru[r + i];
+  }
+  for (int q = tid; q < nnz; q += nt) {
+    av[q] = A.val[q];
+    tv[q] = AT.val[q];
+    ai[q] = A.idx[q];
+    ti[q] = AT.idx[q];
+  }
+  for (int i = tid; i <= m; i += nt) ap[i] = A.ptr[i];
+  for (int j = tid; j <= n; j += nt) tp[j] = AT.ptr[j];
+  __syncthreads();
+  for (int round = 0; round < kIbMaxRounds; ++round) {
+    for (int i = tid; i < m; i += nt) {
+      const RowActivity s = ib_activity(ap[i], ap[i + 1], ai, av, sl, su);
+      alo[i] = s.lo;
+      ahi[i] = s.hi;
+      ilo[i] = s.inf_lo;
+      ihi[i] = s.inf_hi;
+    }
+    __syncthreads();
+    bool moves = false, crosses = false;
+    for (int j = tid; j < n; j += nt) {
+      double l = sl[j], u = su[j];
+      const IbMove move = ib_tighten(tp[j], tp[j + 1], ti, tv, srl, sru, alo, ahi, ilo, ihi, l, u);
+      if (move != kIbCrosses) {
+        sl[j] = l;
+        su[j] = u;
+      }
+      moves = moves || move == kIbMoves;
+      crosses = crosses || move == kIbCrosses;
+    }
+    const bool any_crosses = __syncthreads_or(crosses), any_moves = __syncthreads_or(moves);
+    if (any_crosses || !any_moves) break;
+  }
+  for (int j = tid; j < n; j += nt) {
+    lo[c + j] = sl[j];
+    up[c + j] = su[j];
+  }
+}
+
+// Dynamic shared memory of k_ib_block.
+inline int64_t ib_block_bytes(int64_t m, int64_t n, int64_t nnz) {
+  return 8 * (2 * n + 4 * m + 2 * nnz) + 4 * (2 * m + 2 * nnz + m + n + 2);
+}
+// ... and what a block may have of it (of the device's 227 KB): the block form
+// is taken wherever an LP fits.  Implied bounds of 164 x 324 members, a call
+// with its copies, grid / block form: 1 case 5.80 / 2.22 ms, 61 6.28 / 2.65,
+// 1,024 21.5 / 17.6.  With the operators of a larger LP read from L2 it was
+// no better: 1 case of 1,692 x 3,528 0.60 / 0.77, 61 2.28 / 2.35.
+constexpr int64_t kIbBlockSmem = 224 << 10;
 
 // Device state of the propagation over k cases (case-major bounds, updated in place).
 struct ImpliedBoundsRun {
   int32_t m, n, k;
+  int64_t nnz;
+  bool block;                           // one block a case
   CsrView A, AT;
   const double *rl, *ru;
   double *lo, *up;                      // in: the cases' bounds; out: implied
+  // grid form only
   double *act_lo, *act_hi;              // k x m
   int32_t *inf_lo, *inf_hi;             // k x m
   int32_t* progress;                    // (kIbMaxRounds + 1) x k; row 0 all ones
   int32_t* infeasible;                  // k
 };
 
-// Rounds until no case moves; returns the rounds run.
-inline int run_implied_bounds(cudaStream_t s, const ImpliedBoundsRun& r) {
+// Rounds until no case moves.
+inline void run_implied_bounds(cudaStream_t s, const ImpliedBoundsRun& r) {
+  if (r.m == 0 || r.n == 0) return;
+  if (r.block) {
+    const int threads = std::min(1024, std::max(128, (std::max(r.m, r.n) + 31) / 32 * 32));
+    B2P_CUDA(cudaFuncSetAttribute(k_ib_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kIbBlockSmem)));
+    k_ib_block<<<r.k, threads, static_cast<size_t>(ib_block_bytes(r.m, r.n, r.nnz)), s>>>(
+        r.m, r.n, static_cast<int32_t>(r.nnz), r.A, r.AT, r.rl, r.ru, r.lo, r.up);
+    B2P_CUDA(cudaGetLastError());
+    return;
+  }
   const dim3 grow((r.m + kBlock - 1) / kBlock, r.k), gcol((r.n + kBlock - 1) / kBlock, r.k);
   std::vector<int32_t> ones(r.k, 1), poll(r.k);
   B2P_CUDA(cudaMemcpyAsync(r.progress, ones.data(), sizeof(int32_t) * r.k, cudaMemcpyHostToDevice, s));
   B2P_CUDA(cudaMemsetAsync(r.progress + r.k, 0, sizeof(int32_t) * r.k * kIbMaxRounds, s));
   B2P_CUDA(cudaMemsetAsync(r.infeasible, 0, sizeof(int32_t) * r.k, s));
-  if (r.m == 0 || r.n == 0) {
-    B2P_CUDA(cudaStreamSynchronize(s));
-    return 0;
-  }
   int round = 0;
   while (round < kIbMaxRounds) {
     const int32_t* live = r.progress + static_cast<int64_t>(round) * r.k;
@@ -302,7 +410,6 @@ inline int run_implied_bounds(cudaStream_t s, const ImpliedBoundsRun& r) {
     }
   }
   B2P_CUDA(cudaGetLastError());
-  return round;
 }
 
 // ---- primal checks ---------------------------------------------------------
@@ -490,7 +597,7 @@ inline DeviceOperators upload_operators(CertBuffers& B, const b2p_lp* lp) {
 inline ImpliedBoundsRun make_ib_run(CertBuffers& B, const b2p_lp* lp, int k, const DeviceOperators& ops,
                                     const double* rl, const double* ru, double* lo, double* up) {
   const size_t m = static_cast<size_t>(lp->num_rows);
-  ImpliedBoundsRun r;
+  ImpliedBoundsRun r{};
   r.m = lp->num_rows;
   r.n = lp->num_cols;
   r.k = k;
@@ -500,6 +607,9 @@ inline ImpliedBoundsRun make_ib_run(CertBuffers& B, const b2p_lp* lp, int k, con
   r.ru = ru;
   r.lo = lo;
   r.up = up;
+  r.nnz = lp->start[lp->num_cols];
+  r.block = ib_block_bytes(r.m, r.n, r.nnz) <= kIbBlockSmem;
+  if (r.block) return r;
   r.act_lo = B.get<double>(k * m);
   r.act_hi = B.get<double>(k * m);
   r.inf_lo = B.get<int32_t>(k * m);
