@@ -16,7 +16,7 @@
 // step in the safe direction only when the result was inexact -- so every
 // term, and the in-order sum of each case, is bit-identical to the
 // reference's CPU result.  Cases run in parallel: one thread per column and
-// case for the intervals, one thread per case for the ordered outward sum.
+// case for the intervals, one block per case for the ordered outward sum.
 #include <cuda_runtime.h>
 
 #include <algorithm>
