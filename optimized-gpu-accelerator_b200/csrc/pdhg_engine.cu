@@ -196,7 +196,7 @@ struct Engine {
   int res_blocks = 0, res_gc = 1, res_gr = 1;
   size_t res_smem = 0;
   int32_t *d_cb = nullptr, *d_rb = nullptr;
-  unsigned* d_sync = nullptr;  // arrivals, unused, error flag
+  unsigned* d_sync = nullptr;  // arrivals, error flag
   double* d_rpartial = nullptr;
   int32_t* h_error = nullptr;
   ResidentFn<double> res_fn = nullptr;
@@ -529,7 +529,7 @@ struct Engine {
     const int nb = static_cast<int>(cb.size()) - 1;
     d_cb = upload(cb);
     d_rb = upload(rb);
-    d_sync = dalloc<unsigned>(4);
+    d_sync = dalloc<unsigned>(2);
     d_rpartial = dalloc<double>(static_cast<size_t>(nb) * kNumSums);
     h_error = static_cast<int32_t*>(PinnedCache::get(sizeof(int32_t)));
     *h_error = 0;
@@ -646,13 +646,10 @@ struct Engine {
     ra.ck = IterClock{d_it_base, d_restart_at, 0};
     ra.rho = opt.reflection;
     ra.L = L;
-    ra.g_cols = res_gc;
-    ra.g_rows = res_gr;
     ra.lt_cols = 2 * kResUnroll * res_gc;
     ra.lt_rows = 2 * kResUnroll * res_gr;
     ra.arrive = d_sync;
-    ra.gen = d_sync + 1;
-    ra.error = reinterpret_cast<int32_t*>(d_sync + 2);
+    ra.error = reinterpret_cast<int32_t*>(d_sync + 1);
     ra.partial = d_rpartial;
     // the sums and the outcome go straight to the host's page-locked words
     ra.sums = h_sums;
@@ -781,7 +778,7 @@ struct Engine {
     if (nk) B2P_CUDA(cudaMemsetAsync(v[XP], 0, nk * sizeof(double), stream));
     B2P_CUDA(cudaMemsetAsync(d_it_base, 0, sizeof(int64_t), stream));
     B2P_CUDA(cudaMemsetAsync(d_restart_at, 0, sizeof(int64_t) * k, stream));
-    if (d_sync) B2P_CUDA(cudaMemsetAsync(d_sync, 0, 4 * sizeof(unsigned), stream));
+    if (d_sync) B2P_CUDA(cudaMemsetAsync(d_sync, 0, 2 * sizeof(unsigned), stream));
     res_epoch = 0;
     omega = omega0;
     upload_steps(omega);

@@ -100,15 +100,13 @@ struct ResidentArgs {
   IterClock ck;  // ck.local unused (the kernel walks l = 0..L-1)
   double rho;
   int32_t L;
-  int32_t g_cols, g_rows;      // lanes per short row (A^T, A)
   int32_t lt_cols, lt_rows;    // longer rows go to the warp pass
   // synchronisation and output
   unsigned* arrive;
-  unsigned* gen;
-  int32_t* error;
+  int32_t* error;  // set by a block whose wait timed out, until the next solve
   double* partial;  // gridDim.x * kNumSums
   double* sums;     // kNumSums, page-locked host memory
-  int32_t* failed;  // page-locked host memory: 1 if the interval ended early
+  int32_t* failed;  // page-locked host memory: 1 if any block left the interval early
   int64_t* it_base;
   unsigned epoch0;  // grid barriers of this solve's earlier launches
   int32_t m, n;
@@ -523,7 +521,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(ResidentArgs<T
 #pragma unroll
       for (int q = 0; q < kNumSums; ++q) a.sums[q] = t[q];
       *a.it_base += a.L;
-      *a.failed = ok ? 0 : 1;
+      // a block that gave up at the last dual barrier has brought no check,
+      // yet its arrival here (a release, after it set the word) completes the
+      // count: block 0's own barriers do not tell
+      *a.failed = ok && *reinterpret_cast<volatile int32_t*>(a.error) == 0 ? 0 : 1;
     }
   }
 }
