@@ -37,6 +37,7 @@
 #include "pdhg_slab.cuh"
 #include "pdhg_sched.h"
 #include "pdhg_spmv.cuh"
+#include "pdhg_stop.h"
 #include "pdhg_tiled.cuh"
 
 namespace b2p {
@@ -390,14 +391,9 @@ struct MultiEngine {
   CtaLp* d_lps = nullptr;
   int32_t* d_order = nullptr;
   CtaOut* d_out = nullptr;
-  // Stop flag, read by every block at every check: a device word that the host
-  // sets by a copy on a stream of its own, and only where a deadline or a
-  // cancel flag can set it at all.  (Read from host-mapped memory it cost the
-  // GPU a microsecond per block and check, one after the other over the bus:
-  // 65 ms of the 65 ms of 1,024 small members of 80 checks each.)
-  int32_t* d_stop = nullptr;
-  int32_t* h_one = nullptr;
-  cudaStream_t stop_stream = nullptr;
+  // Stop flag, read by every block at every check; made only where a deadline
+  // or a cancel flag can set it at all.
+  StopWord stop;
   bool may_stop() const { return opt.time_limit > 0 || opt.cancel_flag; }
   // Mixed precision in the CTA form: an FP32 run of every LP (operators and
   // state in FP32), then an FP64 run from each LP's FP32 point.
@@ -454,11 +450,6 @@ struct MultiEngine {
     PinnedCache::put(h_steps, sizeof(double) * 2 * K);
     PinnedCache::put(h_mask, sizeof(int32_t) * K);
     PinnedCache::put(h_done, sizeof(int32_t) * K);
-    if (stop_stream) {
-      cudaStreamSynchronize(stop_stream);
-      cudaStreamDestroy(stop_stream);
-    }
-    PinnedCache::put(h_one, sizeof(int32_t));
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -964,13 +955,7 @@ struct MultiEngine {
     d_order = upload(order);
     host_order = order;
     d_out = dalloc<CtaOut>(K);
-    if (may_stop()) {
-      d_stop = dalloc<int32_t>(1);
-      B2P_CUDA(cudaMemsetAsync(d_stop, 0, sizeof(int32_t), stream));
-      h_one = static_cast<int32_t*>(PinnedCache::get(sizeof(int32_t)));
-      *h_one = 1;
-      B2P_CUDA(cudaStreamCreateWithFlags(&stop_stream, cudaStreamNonBlocking));
-    }
+    if (may_stop()) stop.create(device);
     const int smem = static_cast<int>(cta_smem), osmem = static_cast<int>(cta_owner_smem);
     set_general_attributes<double>(smem);
 #define B2P_OWNER_ATTR(NT, R) \
@@ -1201,7 +1186,7 @@ struct MultiEngine {
     a.entry_check = 0;
     a.stall_checks = 0;
     a.pad = 0;
-    a.stop = d_stop;
+    a.stop = stop.get();
     return a;
   }
 
@@ -1462,7 +1447,7 @@ struct MultiEngine {
         const bool expired = (opt.cancel_flag && *opt.cancel_flag) ||
                              (opt.time_limit > 0 && seconds_since(deadline_start) >= opt.time_limit);
         if (expired && !raised) {
-          B2P_CUDA(cudaMemcpyAsync(d_stop, h_one, sizeof(int32_t), cudaMemcpyHostToDevice, stop_stream));
+          stop.raise();
           raised = true;
         }
         std::this_thread::sleep_for(std::chrono::microseconds(100));
