@@ -47,7 +47,7 @@ namespace b2p {
 
 // Slab-kernel variants: (threads per block, slices of columns and of rows per
 // warp).
-#define B2P_SLAB_VARIANTS(X) X(512, 2, 1) X(512, 4, 2) X(1024, 2, 1)
+#define B2P_SLAB_VARIANTS(X) X(512, 2, 1) X(512, 4, 2)
 // A variant (threads, r) of the CTA form: r <= 0 general, 1 or 2 owner, else
 // slab with r = slab_code(RC, RR).
 constexpr int slab_code(int rc, int rr) { return 100 + 10 * rc + rr; }
