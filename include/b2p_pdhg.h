@@ -153,9 +153,12 @@ typedef struct b2p_options {
    * the kernel variant). */
   int32_t cta_threads;
   /* CTA form: kernel variant (B2P_CTA_*; 0 = autotuned): the general kernel
-   * (any LP size, three storage tiers) or the owner kernel, whose threads
-   * each own 1 or 2 rows and columns and keep their state in registers (LPs
-   * with max(m, n) <= 2 x threads whose data fit in shared memory). */
+   * (any LP size, three storage tiers), the owner kernel, whose threads each
+   * own 1 or 2 rows and columns and keep their state in registers (LPs with
+   * max(m, n) <= 2 x threads whose data fit in shared memory), or the slab
+   * kernel, one LP on a cluster of up to 8 blocks, whose warps hold 2 or 4
+   * slices of 32 columns (LPs whose operators fit those blocks' shared
+   * memory).  A variant that not every LP fits is an error. */
   int32_t cta_kernel;
   /* FP64 batches (k > 1 cases sharing A): variant of the two per-iteration
    * kernels -- 0 = timed on the device when the batch's vectors far exceed L2
@@ -182,7 +185,14 @@ typedef struct b2p_options {
 } b2p_options;
 enum { B2P_CTA_LAYOUT_AUTO = 0, B2P_CTA_LAYOUT_CSR = 1 };
 enum { B2P_MULTI_AUTO = 0, B2P_MULTI_GRID = 1, B2P_MULTI_CTA = 2 };
-enum { B2P_CTA_AUTO = 0, B2P_CTA_GENERAL = 1, B2P_CTA_OWNER1 = 2, B2P_CTA_OWNER2 = 3 };
+enum {
+  B2P_CTA_AUTO = 0,
+  B2P_CTA_GENERAL = 1,
+  B2P_CTA_OWNER1 = 2,
+  B2P_CTA_OWNER2 = 3,
+  B2P_CTA_SLAB2 = 4,
+  B2P_CTA_SLAB4 = 5
+};
 
 enum { B2P_SCHEDULE_AUTO = 0, B2P_SCHEDULE_BINNED = 1, B2P_SCHEDULE_TILED = 2, B2P_SCHEDULE_TUNED = 3 };
 
@@ -190,7 +200,9 @@ enum { B2P_SCHEDULE_AUTO = 0, B2P_SCHEDULE_BINNED = 1, B2P_SCHEDULE_TILED = 2, B
 typedef struct b2p_stats {
   int64_t iterations;
   int32_t restarts;
-  int32_t pad0;
+  /* CTA form: blocks of the cluster that the slab kernel runs each LP on, and
+   * those of the FP32 run (mixed form); 0 = another kernel, one block an LP */
+  int16_t cta_cluster, cta_cluster32;
   double primal_residual, dual_residual, gap;
   double primal_weight;
   double setup_seconds, solve_seconds;
@@ -219,7 +231,7 @@ typedef struct b2p_stats {
   int64_t cta_smem_bytes;                     /* CTA form: dynamic shared memory per block */
   int32_t cta_lps_smem;                       /* CTA form: LPs held wholly in shared memory */
   int32_t cta_lps_vectors;                    /* CTA form: LPs with only their iterates in shared memory */
-  int32_t cta_owned_per_thread;               /* CTA form: rows and columns each thread owns (0 = general kernel) */
+  int32_t cta_owned_per_thread;               /* CTA form: rows and columns each thread owns (0 = general kernel; slab kernel: columns) */
   int32_t tile_rows_at;                       /* FP64 batches: rows per block of the A^T kernel's row-tiled layout (0 = none) */
   int32_t cases_per_thread_at, cases_per_thread_a; /* FP64 batches: cases per thread of the A^T / A kernels */
   int32_t warp_rows_at, warp_rows_a;          /* FP64 batches: whole warps per row, entries shared by shuffle */

@@ -979,6 +979,8 @@ struct MultiEngine {
     stats.cta_lps_smem = n_all;
     stats.cta_lps_vectors = n_vec;
     stats.cta_sliced = d_sa_base != nullptr && cta_r <= 0;
+    stats.cta_cluster = static_cast<int16_t>(cta_r >= 100 ? slab_fit(cta_nt, cta_r, 8).blocks : 0);
+    stats.cta_cluster32 = static_cast<int16_t>(mixed && cta_r32 >= 100 ? slab_fit(cta_nt32, cta_r32, 4).blocks : 0);
   }
 
   // ---- slab kernel (pdhg_slab.cuh) ----
@@ -988,9 +990,11 @@ struct MultiEngine {
     B2P_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     return sms;
   }
-  // Whether the options leave the choice and the batch is one that
-  // slab_candidates can take.
+  bool slab_forced() const { return opt.cta_kernel == B2P_CTA_SLAB2 || opt.cta_kernel == B2P_CTA_SLAB4; }
+  // Whether the options ask for the slab kernel, or leave the choice and the
+  // batch is one that slab_candidates can take.
   bool slab_wanted() const {
+    if (slab_forced()) return true;
     if (opt.cta_kernel != B2P_CTA_AUTO || opt.cta_smem_limit > 0 || opt.cta_layout == B2P_CTA_LAYOUT_CSR) return false;
     bool large = false;
     for (const CtaLp& l : cta_lps) large = large || l.tier != kCtaAll || (mixed && l.tier32 != kCtaAll);
@@ -1017,7 +1021,7 @@ struct MultiEngine {
 #define B2P_SLAB_ANY(NT, RC, RR)                                                        \
   for (const int esize : {8, 4}) {                                                      \
     const int64_t blocks = slab_fit(NT, slab_code(RC, RR), esize).blocks;               \
-    any = any || (blocks > 0 && K * blocks <= sms);                                     \
+    any = any || (blocks > 0 && (slab_forced() || K * blocks <= sms));                  \
   }
     B2P_SLAB_VARIANTS(B2P_SLAB_ANY)
 #undef B2P_SLAB_ANY
@@ -1089,7 +1093,8 @@ struct MultiEngine {
     return found;
   }
 
-  // Slab variants that can run this batch, where the options leave the choice:
+  // Slab variants that can run this batch: any that fits where the options ask
+  // for the slab kernel, else
   // for LPs whose operators do not fit one block (those that do fill the SMs
   // better one block each: 1,024 members of 164 x 324 2.2 ms in either form,
   // 148 0.41 / 0.45), and only while every LP's cluster runs at once (30
@@ -1101,10 +1106,11 @@ struct MultiEngine {
     bool large = false;
     for (const CtaLp& l : cta_lps) large = large || (sizeof(T) == 8 ? l.tier : l.tier32) != kCtaAll;
     const int sms = sm_count();
-    if (!large) return;
+    if (!large && !slab_forced()) return;
 #define B2P_SLAB_CAND(NT, RC, RR)                                                                                  \
   if ((opt.cta_threads == 0 || opt.cta_threads == NT) &&                                                           \
-      static_cast<int64_t>(K) * slab_fit(NT, slab_code(RC, RR), sizeof(T)).blocks <= sms &&                        \
+      (slab_forced() ? opt.cta_kernel == (RC == 4 ? B2P_CTA_SLAB4 : B2P_CTA_SLAB2)                                 \
+                     : static_cast<int64_t>(K) * slab_fit(NT, slab_code(RC, RR), sizeof(T)).blocks <= sms) && \
       launch_slab<T>(NT, slab_code(RC, RR), CtaArgs{}, static_cast<unsigned>(K), true))                            \
     c.emplace_back(NT, slab_code(RC, RR));
     B2P_SLAB_VARIANTS(B2P_SLAB_CAND)
@@ -1264,8 +1270,10 @@ struct MultiEngine {
   // check intervals, twice; the fastest is kept (remembered per batch shape).
   void tune_cta_fp32() {
     const auto t0 = Clock::now();
-    std::vector<std::pair<int, int>> cands = general_candidates();
+    std::vector<std::pair<int, int>> cands;
+    if (!slab_forced()) cands = general_candidates();
     slab_candidates<float>(cands);
+    if (cands.empty()) throw Error(B2P_ERR_INVALID, "no CTA kernel variant fits these LPs and options");
     cta_nt32 = cands.front().first;
     cta_r32 = cands.front().second;
     const int64_t probe = std::min<int64_t>(opt.max_iterations, 5 * static_cast<int64_t>(opt.check_every));
@@ -1345,14 +1353,14 @@ struct MultiEngine {
 
   // Kernel variants that can run this batch: the general kernel at 128, 256,
   // 512 and 1,024 threads (256 and 512 also compiled for 1,024 threads per
-  // SM), and the owner kernel where every LP's rows and columns fit R per
-  // thread and its data fits in shared memory.
+  // SM), the owner kernel where every LP's rows and columns fit R per thread
+  // and its data fits in shared memory, and the slab kernel.
   std::vector<std::pair<int, int>> cta_candidates() {
     const int want = opt.cta_kernel;  // B2P_CTA_*
-    if (want < B2P_CTA_AUTO || want > B2P_CTA_OWNER2) throw Error(B2P_ERR_INVALID, "unknown cta_kernel");
+    if (want < B2P_CTA_AUTO || want > B2P_CTA_SLAB4) throw Error(B2P_ERR_INVALID, "unknown cta_kernel");
     std::vector<std::pair<int, int>> c;
     if (want == B2P_CTA_AUTO || want == B2P_CTA_GENERAL) c = general_candidates();
-    if (cta_owner_smem > 0 && want != B2P_CTA_GENERAL && opt.precision != B2P_PRECISION_MIXED) {
+    if (cta_owner_smem > 0 && want != B2P_CTA_GENERAL && !slab_forced() && opt.precision != B2P_PRECISION_MIXED) {
 #define B2P_OWNER_CAND(NT, R)                                                                        \
   if ((opt.cta_threads == 0 || opt.cta_threads == NT) && cta_max_dim <= NT * R &&                    \
       (want == B2P_CTA_AUTO || want == B2P_CTA_OWNER1 + R - 1))                                      \

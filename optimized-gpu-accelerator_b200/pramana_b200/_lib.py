@@ -23,7 +23,7 @@ KERNELS_AUTO, KERNELS_FUSED, KERNELS_RESIDENT = 0, 1, 2
 SCHEDULE_AUTO, SCHEDULE_BINNED, SCHEDULE_TILED, SCHEDULE_TUNED = 0, 1, 2, 3
 MULTI_AUTO, MULTI_GRID, MULTI_CTA = 0, 1, 2
 CTA_LAYOUT_AUTO, CTA_LAYOUT_CSR = 0, 1
-CTA_AUTO, CTA_GENERAL, CTA_OWNER1, CTA_OWNER2 = 0, 1, 2, 3
+CTA_AUTO, CTA_GENERAL, CTA_OWNER1, CTA_OWNER2, CTA_SLAB2, CTA_SLAB4 = 0, 1, 2, 3, 4, 5
 
 dptr = C.POINTER(C.c_double)
 iptr = C.POINTER(C.c_int32)
@@ -54,9 +54,9 @@ class B2pOptions(C.Structure):
 
 
 class B2pStats(C.Structure):
-    _fields_ = [("iterations", C.c_int64), ("restarts", C.c_int32), ("pad0", C.c_int32),
-                ("primal_residual", C.c_double), ("dual_residual", C.c_double), ("gap", C.c_double),
-                ("primal_weight", C.c_double), ("setup_seconds", C.c_double), ("solve_seconds", C.c_double),
+    _fields_ = [("iterations", C.c_int64), ("restarts", C.c_int32), ("cta_cluster", C.c_int16),
+                ("cta_cluster32", C.c_int16), ("primal_residual", C.c_double), ("dual_residual", C.c_double),
+                ("gap", C.c_double), ("primal_weight", C.c_double), ("setup_seconds", C.c_double), ("solve_seconds", C.c_double),
                 ("kernel_seconds", C.c_double), ("transfer_seconds", C.c_double), ("bytes_uploaded", C.c_int64),
                 ("bytes_downloaded", C.c_int64), ("kernel_launches", C.c_int64), ("spectral_norm", C.c_double),
                 ("prepare_seconds", C.c_double), ("upload_seconds", C.c_double), ("graph_seconds", C.c_double),
