@@ -879,10 +879,16 @@ struct MultiEngine {
 
   // Shared memory one block may give its LP: the device's opt-in per-block
   // maximum less the kernel's static buffers, or the caller's limit.
-  int64_t cta_budget() const {
+  // What the CTA kernels' launches may ask for.  Their limits are set to this,
+  // not to a batch's own need: a limit is the function's, and another thread's
+  // batch may need more.
+  int cta_smem_most() const {
     int optin = 0;
     B2P_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    int64_t b = static_cast<int64_t>(optin) - kCtaStaticReserve;
+    return optin - static_cast<int>(kCtaStaticReserve);
+  }
+  int64_t cta_budget() const {
+    int64_t b = cta_smem_most();
     if (opt.cta_smem_limit > 0) b = std::min<int64_t>(b, opt.cta_smem_limit);
     return std::max<int64_t>(b, 0);
   }
@@ -956,10 +962,10 @@ struct MultiEngine {
     host_order = order;
     d_out = dalloc<CtaOut>(K);
     if (may_stop()) stop.create(device);
-    const int smem = static_cast<int>(cta_smem), osmem = static_cast<int>(cta_owner_smem);
-    set_general_attributes<double>(smem);
+    const int most = cta_smem_most();
+    set_general_attributes<double>(most);
 #define B2P_OWNER_ATTR(NT, R) \
-  B2P_CUDA(cudaFuncSetAttribute(k_lp_owner<NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, osmem));
+  B2P_CUDA(cudaFuncSetAttribute(k_lp_owner<NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     B2P_OWNER_VARIANTS(B2P_OWNER_ATTR)
 #undef B2P_OWNER_ATTR
     mixed = opt.precision == B2P_PRECISION_MIXED;
@@ -1078,7 +1084,7 @@ struct MultiEngine {
 #define B2P_SLAB_LAUNCH(NT, RC, RR)                                                                              \
   if (!found && nt == NT && r == slab_code(RC, RR)) {                                                            \
     const auto fn = k_lp_slab<NT, RC, RR, T>;                                                                    \
-    B2P_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cta_budget()))); \
+    B2P_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cta_smem_most()));              \
     if (probe) {                                                                                                 \
       int clusters = 0;                                                                                          \
       found = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;               \
@@ -1221,7 +1227,7 @@ struct MultiEngine {
     d_ax2 = dalloc<double>(M);
     d_lps2 = dalloc<CtaLp>(K);
     d_order2 = dalloc<int32_t>(K);
-    set_general_attributes<float>(static_cast<int>(cta_smem32));
+    set_general_attributes<float>(cta_smem_most());
   }
   int64_t inst_nnz_total() const {
     int64_t t = 0;
@@ -1233,9 +1239,9 @@ struct MultiEngine {
 // with 1,024 / threads blocks per SM in registers.
 #define B2P_GENERAL_VARIANTS(X) X(128, 0, 1) X(256, 0, 1) X(512, 0, 1) X(1024, 0, 1) X(256, -1, 4) X(512, -1, 2)
   template <class T>
-  void set_general_attributes(int smem) {
+  void set_general_attributes(int most) {
 #define B2P_GEN_ATTR(NT, R, MINB) \
-  B2P_CUDA(cudaFuncSetAttribute(k_lp_cta<NT, T, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  B2P_CUDA(cudaFuncSetAttribute(k_lp_cta<NT, T, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     B2P_GENERAL_VARIANTS(B2P_GEN_ATTR)
 #undef B2P_GEN_ATTR
   }
