@@ -640,10 +640,11 @@ struct MultiEngine {
     B2P_CUDA(cudaGetLastError());
   }
 
-  // Blocks along y for the columns and rows of the largest LP.
-  unsigned member_blocks(bool cols, bool rows) const {
+  // Blocks along y for the columns and rows of the largest of LPs [first,
+  // first + count).
+  unsigned member_blocks(int first, int count, bool cols, bool rows) const {
     int32_t most = 1;
-    for (int b = 0; b < K; ++b) most = std::max(most, std::max(cols ? P[b].n : 0, rows ? P[b].m : 0));
+    for (int b = first; b < first + count; ++b) most = std::max(most, std::max(cols ? P[b].n : 0, rows ? P[b].m : 0));
     return member_grid_y(most);
   }
 
@@ -707,10 +708,11 @@ struct MultiEngine {
     const unsigned k = static_cast<unsigned>(K);
     k_member_raw_sums<<<dim3(k, 4), kOrderedThreads, 0, stream>>>(md, d_msums);
     if (N)
-      k_member_columns<<<dim3(k, member_blocks(true, false)), kBlock, 0, stream>>>(md, d_msums, v[MC], v[MLO], v[MUP],
-                                                                                   v[MXINIT], d_cfac);
+      k_member_columns<<<dim3(k, member_blocks(0, K, true, false)), kBlock, 0, stream>>>(
+          md, d_msums, v[MC], v[MLO], v[MUP], v[MXINIT], d_cfac);
     if (M)
-      k_member_rows<<<dim3(k, member_blocks(false, true)), kBlock, 0, stream>>>(md, d_msums, v[MRL], v[MRU], d_rfac);
+      k_member_rows<<<dim3(k, member_blocks(0, K, false, true)), kBlock, 0, stream>>>(md, d_msums, v[MRL], v[MRU],
+                                                                                      d_rfac);
     k_member_scaled_sums<<<dim3(k, 2), kOrderedThreads, 0, stream>>>(md, v[MC], v[MRL], v[MRU], d_msums);
     B2P_CUDA(cudaGetLastError());
     std::vector<double> sums(static_cast<size_t>(K) * kMemberSums);
@@ -732,8 +734,8 @@ struct MultiEngine {
   // x+ and y+ of LPs [first, first + count) into the answers.
   void take_answers(int first, int count) {
     if (count > 0 && (N || M))
-      k_member_answers<<<dim3(static_cast<unsigned>(count), member_blocks(true, true)), kBlock, 0, stream>>>(
-          md, first, d_msums, v[MXP], v[MYP], d_xans, d_yans);
+      k_member_answers<<<dim3(static_cast<unsigned>(count), member_blocks(first, count, true, true)), kBlock, 0,
+                         stream>>>(md, first, d_msums, v[MXP], v[MYP], d_xans, d_yans);
     B2P_CUDA(cudaGetLastError());
   }
 
