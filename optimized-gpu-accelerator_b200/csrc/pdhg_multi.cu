@@ -1105,9 +1105,11 @@ struct MultiEngine {
   // for the slab kernel, else
   // for LPs whose operators do not fit one block (those that do fill the SMs
   // better one block each: 1,024 members of 164 x 324 2.2 ms in either form,
-  // 148 0.41 / 0.45), and only while every LP's cluster runs at once (30
-  // members of 1,692 x 3,528, 320 iterations, general / slab: 3.2 / 1.2 ms; 296
-  // of them 6.4 / 7.3: the SMs are busy either way).
+  // 148 0.41 / 0.45), and only while their clusters need no more blocks than
+  // there are SMs (30 members of 1,692 x 3,528, 320 iterations, general / slab:
+  // 3.2 / 1.2 ms; 296 of them 6.4 / 7.3: the SMs are busy either way).  Fewer
+  // may run at once -- a cluster's blocks are neighbours, and some SMs are left
+  // over --; the tuning times that too.
   template <class T>
   void slab_candidates(std::vector<std::pair<int, int>>& c) {
     if (!d_slab_cols) return;
@@ -1286,7 +1288,7 @@ struct MultiEngine {
     cta_r32 = cands.front().second;
     const int64_t probe = std::min<int64_t>(opt.max_iterations, 5 * static_cast<int64_t>(opt.check_every));
     if (probe <= 0 || cands.size() == 1) return;
-    const std::vector<int64_t> key{device, K, cta_max_dim, cta_smem32, inst_nnz_total(), opt.check_every,
+    const std::vector<int64_t> key{device, K, ops, cta_max_dim, cta_smem32, inst_nnz_total(), opt.check_every,
                                    opt.cta_threads, opt.cta_kernel, opt.cta_smem_limit, opt.cta_layout};
     static std::mutex mu;
     static std::map<std::vector<int64_t>, std::pair<int, int>> chosen;
@@ -1384,9 +1386,10 @@ struct MultiEngine {
   // Variant choice: each candidate runs every LP for five check intervals
   // (tolerance -1: no LP stops early), twice, and the fastest is kept.  The
   // choice is remembered for the process per batch shape (device, LP count,
-  // largest dimension, shared-memory sizes, nonzeros) and options (the owner
-  // kernel, chosen for a plain batch, cannot run a mixed one's second phase), so repeated
-  // batches of one family pay for it once.
+  // operators -- one that all LPs share stays in L2 --, largest dimension,
+  // shared-memory sizes, nonzeros) and options (the owner kernel, chosen for a
+  // plain batch, cannot run a mixed one's second phase), so repeated batches
+  // of one family pay for it once.
   void tune_cta() {
     const auto t0 = Clock::now();
     if (opt.cta_threads != 0 && opt.cta_threads != 128 && opt.cta_threads != 256 && opt.cta_threads != 512 &&
@@ -1399,8 +1402,8 @@ struct MultiEngine {
     if (probe <= 0 || cands.size() == 1) return;
     int64_t total_nnz = 0;
     for (const CtaLp& c : cta_lps) total_nnz += c.nnz;
-    const std::vector<int64_t> key{device, K, cta_max_dim, cta_smem, cta_owner_smem, total_nnz, opt.cta_threads,
-                                   opt.cta_kernel, opt.check_every, opt.precision, opt.cta_smem_limit,
+    const std::vector<int64_t> key{device, K, ops, cta_max_dim, cta_smem, cta_owner_smem, total_nnz,
+                                   opt.cta_threads, opt.cta_kernel, opt.check_every, opt.precision, opt.cta_smem_limit,
                                    opt.cta_layout};
     static std::mutex mu;
     static std::map<std::vector<int64_t>, std::pair<int, int>> chosen;

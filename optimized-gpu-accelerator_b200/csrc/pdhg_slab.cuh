@@ -29,9 +29,10 @@
 // Measured on 30 members of 1,692 x 3,528 (us per iteration): general kernel
 // 9.9; here 3.7 on clusters of 4 blocks of 512 threads, 5.6 on 2 blocks of
 // 512.  (Blocks of 1,024 threads with two slices a warp hold what 512 with four
-// do, and took 5.9 on 2.)  With members enough to keep every SM busy anyway (296
-// of them) a cluster of 2 takes as long per member and SM as the general
-// kernel, so it serves batches whose clusters all run at once.
+// do, and took 5.9 on 2.)  With members enough to keep every SM busy anyway
+// (296 of them) a cluster of 2 takes as long per member and SM as the general
+// kernel, so it serves batches whose clusters need no more blocks than there
+// are SMs.
 #pragma once
 
 #include <cstdint>
