@@ -262,6 +262,11 @@ int b2p_solve_pdhg(const b2p_lp* lp, const b2p_options* opts, double* x, double*
  * case); results has num_cases entries. */
 int b2p_solve_pdhg_batch(const b2p_lp* base, const b2p_case* cases, int32_t num_cases, const b2p_options* opts,
                          double* x, double* row_dual, b2p_result* results, b2p_stats* batch_stats);
+/* The same with arrays of the cases' own: x[b] and row_dual[b]; either list
+ * or any entry may be NULL. */
+int b2p_solve_pdhg_batch_cases(const b2p_lp* base, const b2p_case* cases, int32_t num_cases, const b2p_options* opts,
+                               double* const* x, double* const* row_dual, b2p_result* results,
+                               b2p_stats* batch_stats);
 
 /* Many independent LPs of different sizes (each with its own A) in one
  * solve.  No counterpart in the reference, which batches only cases sharing
@@ -315,6 +320,9 @@ int b2p_engine_create(const b2p_lp* lp, const b2p_case* cases, int32_t num_cases
                       b2p_engine** out);
 int b2p_engine_solve(b2p_engine* e, b2p_result* results, b2p_stats* stats);
 int b2p_engine_fetch(b2p_engine* e, double* x, double* row_dual);
+/* The same to arrays of the cases' own: x[b] (num_cols) and row_dual[b]
+ * (num_rows); either list or any entry may be NULL. */
+int b2p_engine_fetch_cases(b2p_engine* e, double* const* x, double* const* row_dual);
 int b2p_engine_destroy(b2p_engine* e);
 /* Warm start: the starting point of the following b2p_engine_solve calls, in
  * the original space -- x is num_cases x num_cols, row_dual num_cases x

@@ -1241,6 +1241,56 @@ struct Engine {
     stats.transfer_seconds = transfer_seconds;
   }
 
+  // The same to arrays of the cases' own (NULL entries are skipped), through
+  // page-locked halves: one is filled while the other is dealt out.  (256
+  // cases' 33 MB into one array and copied apart in Python: 25 ms on the host,
+  // 7 so.)
+  static constexpr int64_t kFetchChunk = int64_t(1) << 18;  // doubles
+  void fetch_cases(double* const* x, double* const* y) {
+    if (!solved) return;
+    const auto t0 = Clock::now();
+    B2P_CUDA(cudaSetDevice(device));
+    struct Halves {
+      double* p = static_cast<double*>(PinnedCache::get(2 * kFetchChunk * sizeof(double)));
+      cudaStream_t stream;
+      cudaEvent_t arrived[2] = {nullptr, nullptr};
+      explicit Halves(cudaStream_t s) : stream(s) {}
+      ~Halves() {
+        cudaStreamSynchronize(stream);
+        for (cudaEvent_t e : arrived)
+          if (e) cudaEventDestroy(e);
+        PinnedCache::put(p, 2 * kFetchChunk * sizeof(double));
+      }
+    } halves(stream);
+    for (cudaEvent_t& e : halves.arrived) B2P_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const auto part = [&](const double* src, int64_t len, double* const* dst) {
+      const int64_t total = len * k_full;
+      if (!dst || total == 0) return;
+      const auto send = [&](int64_t at) {
+        const int h = static_cast<int>(at / kFetchChunk & 1);
+        B2P_CUDA(cudaMemcpyAsync(halves.p + h * kFetchChunk, src + at,
+                                 sizeof(double) * std::min(kFetchChunk, total - at), cudaMemcpyDeviceToHost, stream));
+        B2P_CUDA(cudaEventRecord(halves.arrived[h], stream));
+      };
+      send(0);
+      for (int64_t at = 0; at < total; at += kFetchChunk) {
+        if (at + kFetchChunk < total) send(at + kFetchChunk);
+        const int h = static_cast<int>(at / kFetchChunk & 1);
+        B2P_CUDA(cudaEventSynchronize(halves.arrived[h]));
+        const int64_t end = std::min(at + kFetchChunk, total);
+        for (int64_t q = at; q < end;) {
+          const int64_t b = q / len, j = q % len, count = std::min(len - j, end - q);
+          if (dst[b]) std::memcpy(dst[b] + j, halves.p + h * kFetchChunk + (q - at), sizeof(double) * count);
+          q += count;
+        }
+      }
+    };
+    part(d_xans, n, x);
+    part(d_yans, m, y);
+    transfer_seconds += seconds_since(t0);
+    stats.transfer_seconds = transfer_seconds;
+  }
+
   void drop_graphs() {
     for (auto& g : graphs) cudaGraphExecDestroy(g.second);
     for (auto& g : graph_defs) cudaGraphDestroy(g.second);
@@ -1680,6 +1730,13 @@ int b2p_engine_fetch(b2p_engine* h, double* x, double* y) {
   });
 }
 
+int b2p_engine_fetch_cases(b2p_engine* h, double* const* x, double* const* y) {
+  return guarded([&] {
+    if (!h) throw Error(B2P_ERR_INVALID, "engine is NULL");
+    if (x || y) reinterpret_cast<Engine*>(h)->fetch_cases(x, y);
+  });
+}
+
 int b2p_engine_destroy(b2p_engine* h) {
   return guarded([&] { delete reinterpret_cast<Engine*>(h); });
 }
@@ -1735,6 +1792,21 @@ int b2p_solve_pdhg_batch(const b2p_lp* base, const b2p_case* cases, int32_t num_
     e.create(base, cases, num_cases, opts);
     e.solve(t0);
     copy_results(e, x, row_dual, results, batch_stats);
+  });
+}
+
+int b2p_solve_pdhg_batch_cases(const b2p_lp* base, const b2p_case* cases, int32_t num_cases, const b2p_options* opts,
+                               double* const* x, double* const* row_dual, b2p_result* results,
+                               b2p_stats* batch_stats) {
+  return guarded([&] {
+    if (num_cases <= 0) return;
+    if (!cases) throw Error(B2P_ERR_INVALID, "cases is NULL");
+    const auto t0 = b2p::Clock::now();
+    Engine e;
+    e.create(base, cases, num_cases, opts);
+    e.solve(t0);
+    if (x || row_dual) e.fetch_cases(x, row_dual);
+    copy_results(e, nullptr, nullptr, results, batch_stats);
   });
 }
 

@@ -114,6 +114,9 @@ SIGNATURES = {
                                  C.POINTER(B2pStats)]),
     "b2p_solve_pdhg_batch": (C.c_int, [C.POINTER(B2pLp), C.POINTER(B2pCase), C.c_int32, C.POINTER(B2pOptions),
                                        dptr, dptr, C.POINTER(B2pResult), C.POINTER(B2pStats)]),
+    "b2p_solve_pdhg_batch_cases": (C.c_int, [C.POINTER(B2pLp), C.POINTER(B2pCase), C.c_int32, C.POINTER(B2pOptions),
+                                             C.POINTER(dptr), C.POINTER(dptr), C.POINTER(B2pResult),
+                                             C.POINTER(B2pStats)]),
     "b2p_solve_pdhg_multi": (C.c_int, [C.POINTER(B2pLp), C.c_int32, C.POINTER(B2pOptions), C.POINTER(dptr),
                                        C.POINTER(dptr), C.POINTER(dptr), C.POINTER(dptr), C.POINTER(B2pResult),
                                        C.POINTER(B2pStats)]),
@@ -128,6 +131,7 @@ SIGNATURES = {
                                     C.POINTER(C.c_void_p)]),
     "b2p_engine_solve": (C.c_int, [C.c_void_p, C.POINTER(B2pResult), C.POINTER(B2pStats)]),
     "b2p_engine_fetch": (C.c_int, [C.c_void_p, dptr, dptr]),
+    "b2p_engine_fetch_cases": (C.c_int, [C.c_void_p, C.POINTER(dptr), C.POINTER(dptr)]),
     "b2p_engine_destroy": (C.c_int, [C.c_void_p]),
     "b2p_engine_set_profiling": (C.c_int, [C.c_void_p, C.c_int32]),
     "b2p_engine_kernel_times": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int64), dptr]),

@@ -165,6 +165,15 @@ def _address(a) -> int:
     return a.__array_interface__["data"][0]
 
 
+def _answers(lengths):
+    """An array of each length, for an LP's or a case's answer -- of its own, so that keeping one does not keep the
+    whole batch's memory -- and the list of their addresses as C takes it.  A solve that succeeds writes all of each."""
+    arrays = [np.empty(n) for n in lengths]
+    # (a quarter of the time of __array_interface__, which a thousand LPs notice; wants at least one byte)
+    at = np.array([C.addressof(C.c_char.from_buffer(a)) if a.size else 0 for a in arrays], dtype=np.uint64)
+    return arrays, at.ctypes.data_as(C.POINTER(_lib.dptr)), at
+
+
 def _lp_record(lp: Model, keep: list) -> tuple:
     """One LP as a record of _LP_DTYPE.  The arrays the addresses point into
     are Model's own (a copy, kept alive in `keep`, where a field was replaced
@@ -256,17 +265,16 @@ def solvePdhgBatch(base: Model, cases: list[LpCase], opts: PdhgOptions | None = 
     arr, keep2 = _cases_struct(cases, base.num_cols, base.num_rows)
     o = opts.to_c()
     k = len(cases)
-    x = np.zeros(k * base.num_cols)
-    y = np.zeros(k * base.num_rows)
+    xs, xp, keep_x = _answers([base.num_cols] * k)
+    ys, yp, keep_y = _answers([base.num_rows] * k)
     res = (_lib.B2pResult * k)()
     st = _lib.B2pStats()
-    _lib.check(lib.b2p_solve_pdhg_batch(C.byref(s), arr, k, C.byref(o), x.ctypes.data_as(_lib.dptr),
-                                        y.ctypes.data_as(_lib.dptr), res, C.byref(st)))
-    del keep, keep2
+    _lib.check(lib.b2p_solve_pdhg_batch_cases(C.byref(s), arr, k, C.byref(o), xp, yp, res, C.byref(st)))
+    del keep, keep2, keep_x, keep_y
     stats = PdhgStats.from_c(st, _device_name())
     if batchStats is not None:
         batchStats.__dict__.update(stats.__dict__)
-    return _results(res, x.reshape(k, base.num_cols), y.reshape(k, base.num_rows), stats)
+    return _results(res, xs, ys, stats)
 
 
 def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats: PdhgStats | None = None,
@@ -285,14 +293,8 @@ def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats
     k = len(lps)
     keep: list = []
     arr = np.array([_lp_record(lp, keep) for lp in lps], dtype=_LP_DTYPE)
-    # every LP's answer in one buffer, its result a view of it
-    col = np.cumsum([0] + [lp.num_cols for lp in lps])
-    row = np.cumsum([0] + [lp.num_rows for lp in lps])
-    xall, yall = np.zeros(col[-1]), np.zeros(row[-1])
-    xs = [xall[i:j] for i, j in zip(col[:-1].tolist(), col[1:].tolist())]
-    ys = [yall[i:j] for i, j in zip(row[:-1].tolist(), row[1:].tolist())]
-    xp = (_address(xall) + 8 * col[:-1]).astype(np.uint64)
-    yp = (_address(yall) + 8 * row[:-1]).astype(np.uint64)
+    xs, xp, keep_x = _answers([lp.num_cols for lp in lps])
+    ys, yp, keep_y = _answers([lp.num_rows for lp in lps])
     res = (_lib.B2pResult * k)()
     st = _lib.B2pStats()
     o = opts.to_c(cancel_flag)
@@ -308,12 +310,10 @@ def solvePdhgMulti(lps: list[Model], opts: PdhgOptions | None = None, batchStats
         w_in = np.ascontiguousarray(np.asarray(primalWeights, dtype=np.float64).reshape(k))
         keep.append(w_in)
     w_out = np.zeros(k)
-    pp = C.POINTER(_lib.dptr)
     _lib.check(lib.b2p_solve_pdhg_multi_warm(arr.ctypes.data_as(C.POINTER(_lib.B2pLp)), k, C.byref(o), xst, yst,
                                               None if w_in is None else w_in.ctypes.data_as(_lib.dptr),
-                                              xp.ctypes.data_as(pp), yp.ctypes.data_as(pp),
-                                              w_out.ctypes.data_as(_lib.dptr), res, C.byref(st)))
-    del keep
+                                              xp, yp, w_out.ctypes.data_as(_lib.dptr), res, C.byref(st)))
+    del keep, keep_x, keep_y
     stats = PdhgStats.from_c(st, _device_name())
     if batchStats is not None:
         batchStats.__dict__.update(stats.__dict__)
@@ -361,9 +361,11 @@ class Engine:
         st = _lib.B2pStats()
         _lib.check(self._lib.b2p_engine_solve(self._h, res, C.byref(st)))
         self.last_stats = st
-        x, y = self.fetch()
-        return _results(res, x.reshape(self.k, self.lp.num_cols), y.reshape(self.k, self.lp.num_rows),
-                        PdhgStats.from_c(st))
+        xs, xp, keep_x = _answers([self.lp.num_cols] * self.k)
+        ys, yp, keep_y = _answers([self.lp.num_rows] * self.k)
+        _lib.check(self._lib.b2p_engine_fetch_cases(self._h, xp, yp))
+        del keep_x, keep_y
+        return _results(res, xs, ys, PdhgStats.from_c(st))
 
     def set_start(self, x=None, y=None, primal_weight: float = 0.0) -> None:
         """Warm start of the following solves (original space); None, None = cold start."""
