@@ -171,7 +171,7 @@ struct Engine {
   double *d_rscale = nullptr, *d_cscale = nullptr;  // the scaling factors R and Cs
   double *d_xans = nullptr, *d_yans = nullptr;      // answers: num_cases x n / x m, original space
   int32_t* d_ended = nullptr;                       // cases whose answers are taken: packed index, then the engine's
-  bool solved = false;                              // the answers are a solve's
+  bool begun = false;                               // the answers are a solve's (of one that failed: those it got to)
   double* v[NSLOT] = {};
   // Case compaction of a batch (FP64 phase): when half the live cases have
   // terminated, the rest are packed into a narrower interleave, so that the
@@ -1228,9 +1228,10 @@ struct Engine {
     B2P_CUDA(cudaGetLastError());
   }
 
-  // The last solve's answers (none before the first).
+  // The last solve's answers (none before the first; zeros for a case that a
+  // failed one did not get to).
   void fetch(double* x, double* y) {
-    if (!solved) return;
+    if (!begun) return;
     const auto t0 = Clock::now();
     B2P_CUDA(cudaSetDevice(device));
     const size_t nk = static_cast<size_t>(n) * k, mk = static_cast<size_t>(m) * k;
@@ -1247,7 +1248,7 @@ struct Engine {
   // 7 so.)
   static constexpr int64_t kFetchChunk = int64_t(1) << 18;  // doubles
   void fetch_cases(double* const* x, double* const* y) {
-    if (!solved) return;
+    if (!begun) return;
     const auto t0 = Clock::now();
     B2P_CUDA(cudaSetDevice(device));
     struct Halves {
@@ -1380,7 +1381,9 @@ struct Engine {
     int stale32 = 0;
     constexpr int kStallChecks = 20;
     results.assign(k, b2p_result{});
-    solved = false;
+    if (n) B2P_CUDA(cudaMemsetAsync(d_xans, 0, sizeof(double) * n * k, stream));
+    if (m) B2P_CUDA(cudaMemsetAsync(d_yans, 0, sizeof(double) * m * k, stream));
+    begun = true;
     stats.restarts = 0;
     std::vector<char> done(k, 0);
     std::vector<RestartTracker> restarts(k);
@@ -1636,7 +1639,6 @@ struct Engine {
       }
       take_answers(ended);
     }
-    solved = true;
     bytes_down += static_cast<int64_t>(sizeof(double)) * (static_cast<int64_t>(n) + m) * k_full;  // fetch
     stats.kernel_launches = launches;
     stats.bytes_uploaded = bytes_up;
