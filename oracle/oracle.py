@@ -71,7 +71,8 @@ def build(reference: bool = True) -> None:
 
 
 class CheckerMissing(FileNotFoundError, unittest.SkipTest):
-    """A checker's library is not there and cannot be built here: a test that compares with it is skipped."""
+    """The reference's library is not there and neither are its sources: a test that compares with it is skipped.
+    Any other library that is missing is an error."""
 
 
 _libs: dict = {}
@@ -84,7 +85,9 @@ def _load(lib: str):
     if not os.path.exists(path):
         build(reference=(lib == "ref"))
     if not os.path.exists(path):
-        raise CheckerMissing(f"{path} is not built" + ("" if has_reference() else " (no reference sources here)"))
+        if lib == "ref" and not has_reference():
+            raise CheckerMissing(f"{path} is not built, and there are no reference sources here")
+        raise FileNotFoundError(f"{path} is not built")
     h = C.CDLL(path)
     fn = getattr(h, "oracle_pdhg_solve" if lib == "oracle" else "ref_pdhg_solve")
     fn.restype = C.c_int
