@@ -303,12 +303,16 @@ class ErrorWord {
 
 // Buffers of one call on a stream, from the device's stream-ordered pool: a
 // cudaMalloc / cudaFree pair costs 30 us to milliseconds a call and waits for
-// the whole device.
+// the whole device.  The pool keeps what it gets back, so large buffers
+// (training sets, long predictions), whose copies over the bus take far longer
+// than the pair, are allocated and go back to the device with the call.
 class CallBuffers {
  public:
+  static constexpr size_t kPooledMost = size_t(64) << 20;
   CallBuffers(int dev, cudaStream_t stream) : dev_(dev), stream_(stream) {}
   ~CallBuffers() {
-    for (void* p : owned_) cudaFreeAsync(p, stream_);
+    for (void* p : pooled_) cudaFreeAsync(p, stream_);
+    for (void* p : allocated_) cudaFree(p);
   }
   CallBuffers(const CallBuffers&) = delete;
   CallBuffers& operator=(const CallBuffers&) = delete;
@@ -316,15 +320,21 @@ class CallBuffers {
   T* get(size_t count) {
     if (!count) return nullptr;
     void* p = nullptr;
-    B2P_CUDA(cudaMallocFromPoolAsync(&p, count * sizeof(T), device_pool(dev_), stream_));
-    owned_.push_back(p);
+    const size_t bytes = count * sizeof(T);
+    if (bytes <= kPooledMost) {
+      B2P_CUDA(cudaMallocFromPoolAsync(&p, bytes, device_pool(dev_), stream_));
+      pooled_.push_back(p);
+    } else {
+      B2P_CUDA(cudaMalloc(&p, bytes));
+      allocated_.push_back(p);
+    }
     return static_cast<T*>(p);
   }
 
  private:
   int dev_;
   cudaStream_t stream_;
-  std::vector<void*> owned_;
+  std::vector<void*> pooled_, allocated_;
 };
 
 template <class T>
