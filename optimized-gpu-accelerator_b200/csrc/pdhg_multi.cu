@@ -651,31 +651,33 @@ struct MultiEngine {
   // The caller's costs, bounds and sides to the device (through a page-locked
   // buffer filled by all host threads, up to kMemberStage; straight from the
   // caller's arrays beyond), scaled there; the norms and rescaling constants
-  // back (pdhg_members.cuh).
+  // back (pdhg_members.cuh).  The raw arrays lie in iterates, which no solve
+  // has begun to use.
   static constexpr size_t kMemberStage = size_t(128) << 20;
   template <class Parallel>
   void setup_members(const b2p_lp* lps, Parallel&& parallel) {
     const size_t nn = static_cast<size_t>(N), mm = static_cast<size_t>(M);
-    double* d_raw = dalloc<double>(3 * nn + 2 * mm);
-    md.cost = d_raw;
-    md.lower = d_raw + nn;
-    md.upper = d_raw + 2 * nn;
-    md.rl = d_raw + 3 * nn;
-    md.ru = d_raw + 3 * nn + mm;
+    double* const raw[5] = {v[MX], v[MXP], v[MX0], v[MY], v[MYP]};
+    md.cost = raw[0];
+    md.lower = raw[1];
+    md.upper = raw[2];
+    md.rl = raw[3];
+    md.ru = raw[4];
     md.shared = ops != K;
     md.rescale = opt.rescale_objective_and_bounds != 0;
     const size_t bytes = sizeof(double) * (3 * nn + 2 * mm);
     bytes_up += static_cast<int64_t>(bytes);
-    // every array of LP b: its place in the concatenation, its length
+    // every array of LP b: its kind, its place among the kind's, its length
     const auto arrays = [&](int b, auto&& f) {
       const b2p_lp& l = lps[b];
       const size_t c0 = static_cast<size_t>(coff[b]), r0 = static_cast<size_t>(roff[b]);
-      f(c0, l.col_cost, P[b].n);
-      f(nn + c0, l.col_lower, P[b].n);
-      f(2 * nn + c0, l.col_upper, P[b].n);
-      f(3 * nn + r0, l.row_lower, P[b].m);
-      f(3 * nn + mm + r0, l.row_upper, P[b].m);
+      f(0, c0, l.col_cost, P[b].n);
+      f(1, c0, l.col_lower, P[b].n);
+      f(2, c0, l.col_upper, P[b].n);
+      f(3, r0, l.row_lower, P[b].m);
+      f(4, r0, l.row_upper, P[b].m);
     };
+    const size_t begin[6] = {0, nn, 2 * nn, 3 * nn, 3 * nn + mm, 3 * nn + 2 * mm};  // of each kind, in the buffer
     struct Stage {
       double* p = nullptr;
       size_t bytes = 0;
@@ -689,15 +691,19 @@ struct MultiEngine {
     if (bytes > 0 && bytes <= kMemberStage) {
       stage.p = static_cast<double*>(PinnedCache::get(bytes));
       parallel(K, [&](int b) {
-        arrays(b, [&](size_t at, const double* src, int32_t len) {
-          if (len) std::memcpy(stage.p + at, src, sizeof(double) * len);
+        arrays(b, [&](int kind, size_t at, const double* src, int32_t len) {
+          if (len) std::memcpy(stage.p + begin[kind] + at, src, sizeof(double) * len);
         });
       });
-      B2P_CUDA(cudaMemcpyAsync(d_raw, stage.p, bytes, cudaMemcpyHostToDevice, stream));
+      for (int q = 0; q < 5; ++q)
+        if (begin[q + 1] > begin[q])
+          B2P_CUDA(cudaMemcpyAsync(raw[q], stage.p + begin[q], sizeof(double) * (begin[q + 1] - begin[q]),
+                                   cudaMemcpyHostToDevice, stream));
     } else if (bytes > 0) {
       for (int b = 0; b < K; ++b)
-        arrays(b, [&](size_t at, const double* src, int32_t len) {
-          if (len) B2P_CUDA(cudaMemcpyAsync(d_raw + at, src, sizeof(double) * len, cudaMemcpyHostToDevice, stream));
+        arrays(b, [&](int kind, size_t at, const double* src, int32_t len) {
+          if (len)
+            B2P_CUDA(cudaMemcpyAsync(raw[kind] + at, src, sizeof(double) * len, cudaMemcpyHostToDevice, stream));
         });
     }
     d_msums = dalloc<double>(static_cast<size_t>(K) * kMemberSums);
