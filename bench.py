@@ -1239,12 +1239,19 @@ def measured_bf16_peak():
         return 1590.0, "fallback"
 
 
+def gemm_ctas(m, n, sms):
+    """CTAs of k_gemm_group: the widest of its tiles that still give every SM one."""
+    counts = [-(-m // 128) * -(-n // bn) for bn in (256, 128, 64)]
+    return next((c for c in counts[:2] if c >= sms), counts[2])
+
+
 def run_gemm(args, rank, world):
     """--workload gemm: the warm-start network's tcgen05 BF16 GEMM (its TMA form,
-    k_gemm_group: both operands here are K-contiguous) timed with CUDA events (b2p_mlp_gemm_bf16_time) at the network's shapes --
-    batch 1,024 through 512-wide hidden layers, the output layer, a weight
-    gradient (K = batch), the input layer -- and two larger ones, as TFLOP/s
-    of 2 M N K against the bf16 tensor peak."""
+    k_gemm_group: both operands here are K-contiguous) timed with CUDA events
+    (b2p_mlp_gemm_bf16_time) at the network's shapes -- batch 1,024 through
+    512-wide hidden layers, the output layer, a weight gradient (K = batch),
+    the input layer -- and two larger ones, as TFLOP/s of 2 M N K against the
+    bf16 tensor peak."""
     import ctypes as C
 
     import torch
@@ -1255,6 +1262,7 @@ def run_gemm(args, rank, world):
     torch.cuda.set_device(0)
     lib = _lib.load()
     peak, kind = measured_bf16_peak()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     g = torch.Generator(device="cuda").manual_seed(0)
     rows = []
     for m, n, k in GEMM_SHAPES:
@@ -1269,7 +1277,7 @@ def run_gemm(args, rank, world):
         err = float((c - ref).abs().max() / ref.abs().max())
         tflops = 2.0 * m * n * k / (ms.value * 1e-3) / 1e12
         rows.append({"M": m, "N": n, "K": k, "us_per_launch": ms.value * 1e3, "tflops": tflops,
-                     "frac_of_peak": tflops / peak, "ctas": -(-m // 128) * -(-n // 128), "reps": reps,
+                     "frac_of_peak": tflops / peak, "ctas": gemm_ctas(m, n, sms), "reps": reps,
                      "max_rel_err_vs_fp32_matmul": err})
     line = {"metric": "tcgen05 BF16 GEMM TFLOP/s at the warm-start network's shapes", "workload": "gemm",
             "unit": "TFLOP/s", "value": max(r["tflops"] for r in rows), "higher_is_better": True,

@@ -89,9 +89,9 @@ inline cudaMemPool_t device_pool(int dev) {
 
 // Page-locked host buffers, cached for the process: cudaMallocHost pins
 // pages and cudaFreeHost unpins them (and waits for the device), at a cost
-// that varies with the host's load, so the engines take their small pinned
-// buffers (check sums, step sizes, masks, power-iteration vectors) from here
-// and give them back.  Buffers come in power-of-two sizes from 256 bytes; up
+// that varies with the host's load, so the engines take their pinned buffers
+// (check sums, step sizes, masks, power-iteration vectors; up to 128 MB of a
+// call's inputs and answers) from here and give them back.  Buffers come in power-of-two sizes from 256 bytes; up
 // to kPinnedKeepBytes of freed buffers are kept, the rest are freed.
 constexpr size_t kPinnedKeepBytes = size_t(256) << 20;
 
